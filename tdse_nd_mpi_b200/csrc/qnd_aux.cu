@@ -170,72 +170,84 @@ __global__ void __launch_bounds__(256) radial_mask_kernel(const __grid_constant_
     }
 }
 
-// Energy distribution: block b sums, for every energy bin, the Gaussian-weighted densities of its
-// PED_CHUNK elements (those with every |p_j| <= pr_max_j); a second kernel adds the blocks' partial
-// sums in block order (deterministic) and applies the normalisation (io_functions.c:192-199). Bins
-// further than 39 sigma from an element's kinetic energy get exp(...) < 1e-330, which is zero.
+// Flat index and kinetic energy of kept momentum q: the kept set (every |p_j| <= pr_max_j) is a product
+// of per-axis sets, listed in a.kept, so the packed order of the kept momenta is row-major over them.
+__device__ __forceinline__ long long kept_point(const SpectraArgs& a, long long q, double* kin) {
+    long long flat = 0;
+    double e = 0.0;
+    for (int j = 0; j < a.dim; ++j) {
+        const int ij = a.kept[a.axoff[j] + (q / a.stride[j]) % a.npr[j]];
+        flat += (long long)ij << a.shift[j];
+        const double pj = a.p[a.axoff[j] + ij];
+        e += .5 * pj * pj;
+    }
+    if (kin) *kin = e;
+    return flat;
+}
+
+// Energy distribution (io_functions.c:192-199): block b sums, for every energy bin, the Gaussian-weighted
+// densities of its run of a.ped_run kept momenta; a second kernel adds the blocks' partial sums in a
+// fixed order (deterministic) and applies the normalisation. Only kept momenta are visited: at a
+// momentum limit of 2 on a 512^2 grid with spacing 0.2 they are 4,225 of 262,144. Bins further than 39
+// sigma from a kinetic energy get exp(...) < 1e-330, which is zero. The exponentials bound it
+// where many momenta are kept, the length of a block's run where few are (hence short runs).
 template <typename R>
 __global__ void __launch_bounds__(256) ped_partial_kernel(const __grid_constant__ SpectraArgs a, const cplx_t<R>* psi,
                                                           double* partials) {
-    __shared__ double w_s[PED_CHUNK], k_s[PED_CHUNK];
-    const long long i0 = (long long)blockIdx.x * PED_CHUNK;
-    for (int c = threadIdx.x; c < PED_CHUNK; c += blockDim.x) {
-        const long long i = i0 + c;
-        double w = 0.0, kin = 0.0;
-        if (i < a.n) {
-            bool keep = true;
-            for (int j = 0; j < a.dim; ++j) {
-                const long long ij = (i >> a.shift[j]) & a.nmask[j];
-                if (a.rank[a.axoff[j] + ij] < 0) keep = false;
-                const double pj = a.p[a.axoff[j] + ij];
-                kin += .5 * pj * pj;
-            }
-            if (keep) {
-                const cplx_t<R> v = psi[i];
-                const double m = sqrt(double(v.x) * double(v.x) + double(v.y) * double(v.y));
-                w = m * m;
-            }
-        }
-        w_s[c] = w;
-        k_s[c] = kin;
-    }
-    __syncthreads();
+    __shared__ double w_s[PED_TILE], k_s[PED_TILE];
+    const long long q0 = (long long)blockIdx.x * a.ped_run;
+    const long long q1 = q0 + a.ped_run < a.nkept ? q0 + a.ped_run : a.nkept;
     const double inv2s2 = .5 / (a.sigma * a.sigma), reach = 39.0 * a.sigma;
-    for (int j = threadIdx.x; j < a.ne; j += blockDim.x) {
+    for (int j0 = 0; j0 < a.ne; j0 += blockDim.x) {
+        const int j = j0 + threadIdx.x;
         const double e = j * a.de;
         double s = 0.0;
-        for (int c = 0; c < PED_CHUNK; ++c) {
-            const double d = k_s[c] - e;
-            if (w_s[c] != 0.0 && fabs(d) <= reach) s += w_s[c] * exp(-d * d * inv2s2);
+        for (long long t0 = q0; t0 < q1; t0 += PED_TILE) {
+            const int cnt = int(q1 - t0 < PED_TILE ? q1 - t0 : PED_TILE);
+            __syncthreads();  // the tile before is read
+            for (int c = threadIdx.x; c < cnt; c += blockDim.x) {
+                const cplx_t<R> v = psi[kept_point(a, t0 + c, &k_s[c])];
+                const double m = sqrt(double(v.x) * double(v.x) + double(v.y) * double(v.y));
+                w_s[c] = m * m;
+            }
+            __syncthreads();
+            if (j < a.ne)
+                for (int c = 0; c < cnt; ++c) {
+                    const double d = k_s[c] - e;
+                    if (fabs(d) <= reach) s += w_s[c] * exp(-d * d * inv2s2);
+                }
         }
-        partials[(long long)blockIdx.x * a.ne + j] = s;
+        if (j < a.ne) partials[(long long)blockIdx.x * a.ne + j] = s;
     }
 }
 
-__global__ void ped_final_kernel(const __grid_constant__ SpectraArgs a, const double* partials, int nblocks, double* out) {
-    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < a.ne; j += gridDim.x * blockDim.x) {
-        double s = 0.0;
-        for (int b = 0; b < nblocks; ++b) s += partials[(long long)b * a.ne + j];
+// One energy bin per thread column: 32 threads of a column each add every 32nd block's partial sum, the
+// first of them adds the 32 sums in order. One thread per bin adding all blocks took 169 us at 1024
+// blocks and 400 bins, a chain of one load after the other; the columns take 5 us there.
+__global__ void __launch_bounds__(1024) ped_final_kernel(const __grid_constant__ SpectraArgs a, const double* partials,
+                                                         int nblocks, double* out) {
+    __shared__ double part[32][33];
+    const int jl = threadIdx.x & 31, row = threadIdx.x >> 5;
+    const int j = blockIdx.x * 32 + jl;
+    double s = 0.0;
+    if (j < a.ne)
+        for (int b = row; b < nblocks; b += 32) s += partials[(long long)b * a.ne + j];
+    part[row][jl] = s;
+    __syncthreads();
+    if (row == 0 && j < a.ne) {
+        for (int r = 1; r < 32; ++r) s += part[r][jl];
         out[j] = s * a.norm;
     }
 }
 
 // Momentum distribution: (|psi~|^2, arg psi~) of the kept momenta, packed in flat order
-// (io_functions.c:266-274); the kept set is a product of per-axis sets, so an element's place in the
-// packed array follows from its per-axis ranks.
+// (io_functions.c:266-274).
 template <typename R>
 __global__ void __launch_bounds__(256) pmd_kernel(const __grid_constant__ SpectraArgs a, const cplx_t<R>* psi,
                                                   double* out) {
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < a.n; i += (long long)gridDim.x * blockDim.x) {
-        long long q = 0;
-        bool keep = true;
-        for (int j = 0; j < a.dim; ++j) {
-            const int rk = a.rank[a.axoff[j] + ((i >> a.shift[j]) & a.nmask[j])];
-            if (rk < 0) keep = false;
-            q += (long long)rk * a.stride[j];
-        }
-        if (!keep) continue;
-        const cplx_t<R> v = psi[i];
+    for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < a.nkept;
+         q += (long long)gridDim.x * blockDim.x) {
+        const cplx_t<R> v = psi[kept_point(a, q, nullptr)];
         const double re = v.x, im = v.y;
         const double m = sqrt(re * re + im * im);
         out[2 * q] = m * m;
@@ -251,14 +263,14 @@ void launch_radial_mask(const SpectraArgs& a, const cplx_t<R>* in, cplx_t<R>* ou
 }
 template <typename R>
 void launch_ped(const SpectraArgs& a, const cplx_t<R>* psi_p, double* partials, double* out, cudaStream_t st) {
-    const int nb = int((a.n + PED_CHUNK - 1) / PED_CHUNK);
-    ped_partial_kernel<R><<<nb, 256, 0, st>>>(a, psi_p, partials);
-    ped_final_kernel<<<(a.ne + 255) / 256, 256, 0, st>>>(a, partials, nb, out);
+    const int nb = ped_blocks(a);
+    if (nb) ped_partial_kernel<R><<<nb, 256, 0, st>>>(a, psi_p, partials);
+    ped_final_kernel<<<(a.ne + 31) / 32, 1024, 0, st>>>(a, partials, nb, out);
 }
 template <typename R> void launch_pmd(const SpectraArgs& a, const cplx_t<R>* psi_p, double* out, cudaStream_t st) {
-    long long nb = (a.n + 255) / 256;
+    long long nb = (a.nkept + 255) / 256;
     if (nb > 148 * 16) nb = 148 * 16;
-    pmd_kernel<R><<<(int)nb, 256, 0, st>>>(a, psi_p, out);
+    if (nb) pmd_kernel<R><<<(int)nb, 256, 0, st>>>(a, psi_p, out);
 }
 
 // ---- laser field samples (integrators.c:74-101, parameters.c:899-949) -------------

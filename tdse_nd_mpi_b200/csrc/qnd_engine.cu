@@ -185,7 +185,7 @@ struct qnd_ctx {
     std::vector<RecordedPass>* recorder = nullptr;
     const void* field_view = nullptr;
     DevBuf sweep_field, sweep_buf;
-    DevBuf spec_rank, spec_partials, spec_out;  // final spectra: per-axis ranks, partial sums, results
+    DevBuf spec_kept, spec_partials, spec_out;  // final spectra: kept momenta per axis, partial sums, results
     DevBuf field_out, embed_src;                // qnd_field_samples host-output staging; qnd_state_embed source
     DevBuf err_flag;                            // set by a kernel whose bounded wait ran out
     DevBuf tune_buf;                            // scratch state of the staging autotuner
@@ -3262,22 +3262,22 @@ int qnd_final_spectra(qnd_ctx* ctx, const void* psi_r_dev, double r_mask_min, do
     if (!(r_mask_max > r_mask_min)) QND_FAIL(QND_EINVAL, "qnd_final_spectra: R_MASK needs Rmin < Rmax");
     set_device(ctx);
     const int d = ctx->dim;
-    // kept momenta per axis (|p| <= pr_max, io_functions.c:191, :218-225) and their ranks
-    std::vector<int> rank(size_t(ctx->axtot), -1);
+    // kept momenta per axis (|p| <= pr_max, io_functions.c:191, :218-225)
+    std::vector<int> kept(size_t(ctx->axtot), 0);
     int64_t npr[MAX_DIM] = {};
     for (int j = 0; j < d; ++j)
         for (int k = 0; k < int(ctx->nr[j]); ++k)
-            if (std::fabs(ctx->p[j][k]) <= pr_max[j]) rank[ctx->axoff[j] + k] = int(npr[j]++);
+            if (std::fabs(ctx->p[j][k]) <= pr_max[j]) kept[ctx->axoff[j] + npr[j]++] = k;
     if (npr_host)
         for (int j = 0; j < d; ++j) npr_host[j] = npr[j];
     if (!ped_host && !pmd_host) return QND_OK;
-    ctx->spec_rank.ensure(rank.size() * sizeof(int));
-    QND_CK(cudaMemcpyAsync(ctx->spec_rank.p, rank.data(), rank.size() * sizeof(int), cudaMemcpyHostToDevice,
+    ctx->spec_kept.ensure(kept.size() * sizeof(int));
+    QND_CK(cudaMemcpyAsync(ctx->spec_kept.p, kept.data(), kept.size() * sizeof(int), cudaMemcpyHostToDevice,
                            ctx->stream));
     SpectraArgs a{};
     a.r = ctx->r_dev.as<double>();
     a.p = ctx->p_dev.as<double>();
-    a.rank = ctx->spec_rank.as<int>();
+    a.kept = ctx->spec_kept.as<int>();
     a.dim = d;
     a.n = ctx->n;
     long long stride = 1;
@@ -3289,7 +3289,10 @@ int qnd_final_spectra(qnd_ctx* ctx, const void* psi_r_dev, double r_mask_min, do
         a.axoff[j] = ctx->axoff[j];
         a.shift[j] = ctx->shift[j];
         a.nmask[j] = ctx->nr[j] - 1;
+        a.npr[j] = npr[j];
     }
+    a.nkept = stride;
+    a.ped_run = ped_run(stride);
     a.rmin = r_mask_min;
     a.rmax = r_mask_max;
     a.de = de;
@@ -3307,8 +3310,7 @@ int qnd_final_spectra(qnd_ctx* ctx, const void* psi_r_dev, double r_mask_min, do
     QND_CK(cudaGetLastError());
     unitary_fft(ctx, q, true);
     if (ped_host) {
-        const size_t nb = size_t((ctx->n + PED_CHUNK - 1) / PED_CHUNK);
-        ctx->spec_partials.ensure(nb * size_t(ne) * sizeof(double));
+        ctx->spec_partials.ensure(size_t(ped_blocks(a)) * size_t(ne) * sizeof(double));
         ctx->spec_out.ensure(size_t(ne) * sizeof(double));
         if (ctx->fp64)
             launch_ped<double>(a, static_cast<const double2*>(q), ctx->spec_partials.as<double>(),

@@ -116,7 +116,10 @@ template <typename R> void launch_axis_table(int mode, const double* p, int N, d
 struct SpectraArgs {
     const double* r;      // concatenated r axes
     const double* p;      // concatenated p axes (FFT order)
-    const int* rank;      // concatenated per-axis rank among the kept momenta (|p| <= pr_max), -1 if not kept
+    const int* kept;      // per axis (at axoff) the indices of its kept momenta (|p| <= pr_max), ascending
+    long long npr[MAX_DIM];  // kept momenta per axis
+    long long nkept;         // their product
+    long long ped_run;       // kept momenta per block of the energy distribution
     int axoff[MAX_DIM];
     int shift[MAX_DIM];
     long long nmask[MAX_DIM];
@@ -127,7 +130,14 @@ struct SpectraArgs {
     double de, sigma, norm;
     int ne;
 };
-constexpr int PED_CHUNK = 256;  // elements per block of the energy-distribution partial sums
+constexpr int PED_TILE = 256;  // kept momenta a block of the energy distribution holds at a time
+// Kept momenta per block: 16 while that gives at most 592 blocks (4 per SM), so that few kept momenta
+// still spread over the SMs, then as many as 592 blocks need.
+inline long long ped_run(long long nkept) {
+    const long long per = (nkept + 591) / 592;
+    return per < 16 ? 16 : per;
+}
+inline int ped_blocks(const SpectraArgs& a) { return int((a.nkept + a.ped_run - 1) / a.ped_run); }
 template <typename R>
 void launch_radial_mask(const SpectraArgs& a, const cplx_t<R>* in, cplx_t<R>* out, cudaStream_t st);
 template <typename R>

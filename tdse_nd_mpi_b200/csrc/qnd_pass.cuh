@@ -334,15 +334,25 @@ __device__ __forceinline__ void accumulate_line(const RedDesc& rd, double* acc, 
                 sum *= wl;
             }
         } else {
+            // the weights' row and their step along it, or no weights (one branch for the whole line)
+            const double* __restrict__ row = nullptr;
+            int step = T;
+            if (wk == WK_GRID) {
+                row = wt + lbase + tid;
+            } else if (wk == WK_AXIS) {
+                if (rd.waxis[k] == axis) row = wt + tid;
+                else { row = wt + ((base >> rd.wshift[k]) & rd.wmask[k]); step = 0; }
+            }
+            auto bilin = [&](int u) {
+                const cplx_t<R> p = partner[base + ((long long)(tid + u * T) << log2S)];
+                return double(p.x) * double(v[u].x) + double(p.y) * double(v[u].y);
+            };
+            if (row) {
 #pragma unroll
-            for (int u = 0; u < E; ++u) {
-                const int m = tid + u * T;
-                const long long flat = base + ((long long)m << log2S);
-                const cplx_t<R> p = partner[flat];
-                double val = double(p.x) * double(v[u].x) + double(p.y) * double(v[u].y);
-                if (wk == WK_AXIS) val *= __ldg(wt + ((flat >> rd.wshift[k]) & rd.wmask[k]));
-                else if (wk == WK_GRID) val *= __ldg(wt + lbase + m);
-                sum += val;
+                for (int u = 0; u < E; ++u) sum += bilin(u) * __ldg(row + u * step);
+            } else {
+#pragma unroll
+                for (int u = 0; u < E; ++u) sum += bilin(u);
             }
         }
         acc[k] += sum;
@@ -765,18 +775,17 @@ __device__ __forceinline__ void pass_group(const PassArgs<R>& a, long long g, un
                                            a.shift, a.nmask, nullptr, key0 ^ 0x68e31da4u);
                 if (HAS_RED && a.red.n && !a.red_at_mid)
                     accumulate_line<R, E, T>(a.red, acc, v, a.partner, base, log2S, lbase, tid, a.axis, a.shift, a.nmask);
-            } else {  // PM_APPLY
+            } else {  // PM_APPLY: a branch-free loop per term, so that its reads go out together
+                auto flat_at = [&](int u) { return base + ((long long)(tid + u * T) << log2S); };
+                if (a.apply_vtab) {
 #pragma unroll
-                for (int u = 0; u < E; ++u) {
-                    const long long flat = base + ((long long)(tid + u * T) << log2S);
-                    V x = v[u];
-                    if (a.apply_vtab) {
-                        const V p = a.psi[flat];
-                        const R vv = R(a.apply_vtab[flat]);
-                        x = cadd(x, cscale(p, vv));
-                    }
-                    if (a.apply_acc) x = cadd(x, a.dst[flat]);
-                    v[u] = x;
+                    for (int u = 0; u < E; ++u)
+                        v[u] = cadd(v[u], cscale(a.psi[flat_at(u)], R(__ldg(a.apply_vtab + flat_at(u)))));
+                }
+                if (a.apply_acc) {
+                    const V* __restrict__ sum = a.dst;
+#pragma unroll
+                    for (int u = 0; u < E; ++u) v[u] = cadd(v[u], sum[flat_at(u)]);
                 }
                 if (a.red.n)
                     accumulate_line<R, E, T>(a.red, acc, v, a.partner, base, log2S, lbase, tid, a.axis, a.shift, a.nmask);
