@@ -297,11 +297,11 @@ static void round_pairs_f32_balanced(const double* v, size_t n, float* out) {
     }
 }
 
-// Stage twiddles of HostPlan(L), exp(-2 pi i jm r / (Ns R)) in long double: FP64 plans one base per
-// butterfly position (r = 1; the kernel forms the powers, pow_twiddles), FP32 plans every r in the
+// Stage twiddles of HostPlan(L) (for E values per thread, default the pass kernels'), exp(-2 pi i jm r / (Ns R)) in long double: FP64 plans one base per
+// butterfly position (r = 1; the kernel forms the powers, TwiddledDFT), FP32 plans every r in the
 // [j mod Ns][r-1] layout.
-static void build_twiddles(qnd_ctx* c, int L, DevBuf& dst) {
-    HostPlan pl(L, lookup_pass(c->fp64, L, false, PM_SANDWICH).E);
+static void build_twiddles(qnd_ctx* c, int L, DevBuf& dst, int E = 0) {
+    HostPlan pl(L, E ? E : lookup_pass(c->fp64, L, false, PM_SANDWICH).E);
     const int entries = c->fp64 ? pl.twb_size : pl.tw_size;
     std::vector<double> tw(2 * size_t(entries > 0 ? entries : 1));
     const long double two_pi = 6.283185307179586476925286766559005768L;

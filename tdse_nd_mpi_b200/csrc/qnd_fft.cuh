@@ -165,14 +165,43 @@ template <int N, int K, int SIGN, typename V> __device__ __forceinline__ V twidd
     }
 }
 
+// p = a + c b, m = a - c b in six fused multiply-adds: m as 2a - p (exact up to its own rounding and
+// p's), where forming c b first takes eight operations.
+template <typename V> __device__ __forceinline__ void butterfly(V a, V b, V c, V& p, V& m) {
+    p.x = fma(c.x, b.x, fma(-c.y, b.y, a.x));
+    p.y = fma(c.x, b.y, fma(c.y, b.x, a.y));
+    m.x = fma(decltype(a.x)(2), a.x, -p.x);
+    m.y = fma(decltype(a.y)(2), a.y, -p.y);
+}
+
+// exp(SIGN * 2*pi*i*K/N), N <= 32 and K < N/4.
+template <int N, int K, int SIGN, typename V> __device__ __forceinline__ constexpr V root_const() {
+    static_assert(32 % N == 0 && 4 * K < N, "root_const: the first quarter of N <= 32 roots");
+    constexpr int e = K * (32 / N);
+    return V{cos_pi16(e), SIGN * cos_pi16(8 - e)};
+}
+
+// b times exp(SIGN * i*pi/2).
+template <int SIGN, typename V> __device__ __forceinline__ V quarter_turn(V b) {
+    if constexpr (SIGN > 0) return V{-b.y, b.x};
+    else return V{b.y, -b.x};
+}
+
 // In-register R-point DFT (natural order in and out), radix-2 decimation in time.
 template <int R, int SIGN> struct RegDFT {
     template <typename V, int... K>
     __device__ __forceinline__ static void combine(V* v, const V* e, const V* o, std::integer_sequence<int, K...>) {
         ((void)([&] {
-             V t = twiddle_const<R, K, SIGN>(o[K]);
-             v[K] = cadd(e[K], t);
-             v[K + R / 2] = csub(e[K], t);
+             constexpr bool trivial = 4 * K % R == 0;
+             if constexpr (sizeof(e[0].x) == 8 && !trivial) {
+                 constexpr int k = 4 * K < R ? K : K - R / 4;  // a quarter turn and a root of the first quarter
+                 butterfly(e[K], k == K ? o[K] : quarter_turn<SIGN>(o[K]), root_const<R, k, SIGN, V>(), v[K],
+                           v[K + R / 2]);
+             } else {
+                 V t = twiddle_const<R, K, SIGN>(o[K]);
+                 v[K] = cadd(e[K], t);
+                 v[K + R / 2] = csub(e[K], t);
+             }
          }()),
          ...);
     }
@@ -219,7 +248,7 @@ template <int L, int E> struct FFTPlan {
     }
     __host__ __device__ static constexpr int tw_size() { return tw_offset(NSTAGE) ; }
     // FP64 plans store one base twiddle per butterfly position, W_{Ns R}^{jm} for jm < Ns, and form
-    // its powers in registers (pow_twiddles): stage st's bases start at twb_offset(st)
+    // its powers in registers (TwiddledDFT): stage st's bases start at twb_offset(st)
     __host__ __device__ static constexpr int twb_offset(int st) {
         return st <= 1 ? 0 : twb_offset(st - 1) + span(st - 1);
     }
@@ -227,30 +256,39 @@ template <int L, int E> struct FFTPlan {
     static constexpr int SMEM_LINE = L + L / E;  // padded values per line (before line padding)
 };
 
-// Multiply u[1..R-1] by w^1 .. w^(R-1) with w the base twiddle of the butterfly (FP64 plans). The
-// powers are formed as w^(4k + j) = w^(4k) w^j from w, w^2, w^3 and the running w^(4k) (w^4, w^8 =
-// (w^4)^2, w^12 = w^8 w^4): at most four rounded products deep, about four units in the last place,
-// against one shared-memory load per twiddle in the table form. Trades shared-memory bandwidth, the
-// bound of the transform's exchanges, for FP64 multiplies.
-template <int R, typename V> __device__ __forceinline__ void pow_twiddles(V* u, V w) {
-    if constexpr (R >= 2) u[1] = cmul(u[1], w);
-    if constexpr (R >= 4) {
-        const V w2 = cmul(w, w);
-        const V w3 = cmul(w2, w);
-        u[2] = cmul(u[2], w2);
-        u[3] = cmul(u[3], w3);
-        const V w4 = cmul(w2, w2);
-        V w4k = w4;
-#pragma unroll
-        for (int k = 1; k < R / 4; ++k) {
-            u[4 * k] = cmul(u[4 * k], w4k);
-            u[4 * k + 1] = cmul(u[4 * k + 1], cmul(w4k, w));
-            u[4 * k + 2] = cmul(u[4 * k + 2], cmul(w4k, w2));
-            u[4 * k + 3] = cmul(u[4 * k + 3], cmul(w4k, w3));
-            if (k + 1 < R / 4) w4k = (k == 1) ? cmul(w4, w4) : cmul(w4k, w4);
-        }
+// R-point DFT of v[r] w^r (natural order in and out, FP64 plans): the stage twiddles are taken into the
+// butterflies. At the level that joins two DFTs of size R/2 the factor of output k is w W_R^k, and the
+// halves are the same problem with w^2, so a radix-16 stage has eight distinct complex factors (up to
+// quarter turns) formed from one base w by three squarings and four products with constants: 192 fused
+// multiply-adds and 28 operations for the factors, where multiplying by w .. w^15 first (powers formed
+// from the same base) and then transforming took 168 + 116. A 1024-point transform falls from 596 to 480
+// FP64 instructions per 16 points. pw: w, w^2, w^4, ... (R / 2 and on).
+template <int R, int SIGN> struct TwiddledDFT {
+    template <typename V, int... K>
+    __device__ __forceinline__ static void combine(V* v, const V* e, const V* o, V w, std::integer_sequence<int, K...>) {
+        ((void)([&] {
+             constexpr bool turn = R >= 4 && 4 * K >= R;
+             constexpr int k = turn ? K - R / 4 : K;
+             V c = w;
+             if constexpr (k > 0) c = cmul(w, root_const<R, k, SIGN, V>());
+             butterfly(e[K], turn ? quarter_turn<SIGN>(o[K]) : o[K], c, v[K], v[K + R / 2]);
+         }()),
+         ...);
     }
-}
+    template <typename V> __device__ __forceinline__ static void run(V* v, const V* pw) {
+        V e[R / 2], o[R / 2];
+#pragma unroll
+        for (int i = 0; i < R / 2; ++i) {
+            e[i] = v[2 * i];
+            o[i] = v[2 * i + 1];
+        }
+        if constexpr (R > 2) {
+            TwiddledDFT<R / 2, SIGN>::run(e, pw + 1);
+            TwiddledDFT<R / 2, SIGN>::run(o, pw + 1);
+        }
+        combine(v, e, o, pw[0], std::make_integer_sequence<int, R / 2>{});
+    }
+};
 
 // One Stockham stage on the thread's E registers (B = E/R butterflies, j = tid + b*T).
 // Input registers hold x[j + r*L/R] for butterfly b at v[b*R + r]; output registers hold
@@ -275,7 +313,12 @@ __device__ __forceinline__ void fft_stage_regs(V* v, int tid, const V* __restric
                 if constexpr (TWS) w = *t;
                 else w = __ldg(t);
                 if constexpr (SIGN > 0) w.y = -w.y;
-                pow_twiddles<R>(u, w);
+                V pw[ilog2(R)];
+                pw[0] = w;
+#pragma unroll
+                for (int q = 1; q < ilog2(R); ++q) pw[q] = cmul(pw[q - 1], pw[q - 1]);
+                TwiddledDFT<R, SIGN>::run(u, pw);
+                continue;
             } else {
                 const V* t = tw + P::tw_offset(ST) + jm * (R - 1);
 #pragma unroll

@@ -161,7 +161,7 @@ template <typename R, int L, int VAR = 0> struct PassShape {
     static constexpr int LS_TARGET = G >= SLOTS ? 1 : SLOTS / G;
     static constexpr int LINE_RAW = FFTPlan<L, E>::SMEM_LINE;
     static constexpr int LS = LINE_RAW + ((LS_TARGET - LINE_RAW % SLOTS) % SLOTS + SLOTS) % SLOTS;
-    // stage twiddle entries: FP64 plans keep one base per butterfly position (pow_twiddles)
+    // stage twiddle entries: FP64 plans keep one base per butterfly position (TwiddledDFT)
     static constexpr int TW_ENTRIES = sizeof(R) == 8 ? FFTPlan<L, E>::twb_size() : FFTPlan<L, E>::tw_size();
     static constexpr int TWN_RAW = (TW_ENTRIES + 1) & ~1;
     // stage twiddles in shared memory when they are small and shared by several lines of the CTA;
