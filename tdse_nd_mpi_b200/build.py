@@ -49,6 +49,9 @@ def _jobs():
     for fp64 in (1, 0):
         jobs.insert(0, (os.path.join(CSRC, "qnd_sweep.cu"), os.path.join(BUILD, f"qnd_sweep_fp{64 if fp64 else 32}.o"),
                         [f"-DQND_SWEEP_FP64={fp64}"]))
+    for fp64 in (1, 0):
+        jobs.append((os.path.join(CSRC, "qnd_chain1d.cu"), os.path.join(BUILD, f"qnd_chain1d_fp{64 if fp64 else 32}.o"),
+                     [f"-DQND_CHAIN_FP64={fp64}"]))
     return jobs
 
 

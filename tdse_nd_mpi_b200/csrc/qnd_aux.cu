@@ -406,14 +406,16 @@ __global__ void __launch_bounds__(256) long_transpose_kernel(LongArgs a, const c
 
 template <typename R>
 __global__ void __launch_bounds__(256) point_factors_kernel(long long n, cplx_t<R>* psi, const R* tr,
-                                                            const cplx_t<R>* tc, const cplx_t<R>* pc, const R* pr,
-                                                            const double* scale_dev) {
+                                                            const cplx_t<R>* tc, const cplx_t<R>* pc, LongArgs pc_order,
+                                                            const R* pr, const double* scale_dev) {
     const R sc = scale_dev ? R(*scale_dev) : R(1);
+    const long long m2 = (1ll << pc_order.log2n2) - 1;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         cplx_t<R> x = psi[i];
         if (tr) x = cscale(x, tr[i]);
         if (tc) x = fmul(x, tc[i]);
-        if (pc) x = fmul(x, pc[i]);
+        // the laser phases: line-major for the strided virtual axis
+        if (pc) x = fmul(x, pc[((i & m2) << pc_order.log2n1) + (i >> pc_order.log2n2)]);
         if (pr) x = cscale(x, pr[i]);
         if (scale_dev) x = cscale(x, sc);
         psi[i] = x;
@@ -516,9 +518,9 @@ template <typename R> void launch_long_transpose(const LongArgs& a, const cplx_t
     long_transpose_kernel<R><<<elementwise_blocks(a.n), 256, 0, st>>>(a, in, out, to_natural);
 }
 template <typename R> void launch_point_factors(long long n, cplx_t<R>* psi, const R* tr, const cplx_t<R>* tc,
-                                                const cplx_t<R>* pc, const R* pr, const double* scale_dev,
-                                                cudaStream_t st) {
-    point_factors_kernel<R><<<elementwise_blocks(n), 256, 0, st>>>(n, psi, tr, tc, pc, pr, scale_dev);
+                                                const cplx_t<R>* pc, const LongArgs& pc_order, const R* pr,
+                                                const double* scale_dev, cudaStream_t st) {
+    point_factors_kernel<R><<<elementwise_blocks(n), 256, 0, st>>>(n, psi, tr, tc, pc, pc_order, pr, scale_dev);
 }
 template <typename R> void launch_apply_masks(long long n, cplx_t<R>* psi, int dim, const int* shift,
                                               const long long* nmask, const R* const* masks, cudaStream_t st) {
@@ -561,7 +563,7 @@ template <typename R> void launch_apply_combine(long long n, cplx_t<R>* dst, con
     template void launch_long_twiddle<R>(const LongArgs&, cplx_t<R>*, const cplx_t<R>*, int, cudaStream_t); \
     template void launch_long_transpose<R>(const LongArgs&, const cplx_t<R>*, cplx_t<R>*, int, cudaStream_t); \
     template void launch_point_factors<R>(long long, cplx_t<R>*, const R*, const cplx_t<R>*, const cplx_t<R>*, \
-                                          const R*, const double*, cudaStream_t);                          \
+                                          const LongArgs&, const R*, const double*, cudaStream_t);         \
     template void launch_add_potential<R>(long long, cplx_t<R>*, const cplx_t<R>*, const double*, cudaStream_t); \
     template void launch_embed<R>(const EmbedArgs&, const double2*, cplx_t<R>*, cudaStream_t);                \
     template void launch_apply_masks<R>(long long, cplx_t<R>*, int, const int*, const long long*, const R* const*, \

@@ -1,0 +1,183 @@
+// qnd_chain1d.cu — a whole chain of kinetic sandwiches on a 1-D grid of up to 4096 points in one
+// launch: one CTA holds the line in registers from the first sandwich to the last, so that a chain
+// reads and writes the state once and pays one launch, instead of one pass of one CTA per pair of
+// sandwiches with the launches, the state's round trip through L2 and (imaginary time) the
+// Gram-Schmidt kernels between them.
+//
+// What bounds it: one SM. A line of 4096 FP64 points needs 588 FP64 instructions per 16 points and
+// transform, about 2,400 cycles of one SM's FP64 pipe, and its exchanges about 2,000 cycles of its
+// shared memory; two transforms per sandwich. The tables come from L2, read into registers before the
+// transform that precedes their use.
+#include "qnd_kernels.cuh"
+
+#ifndef QND_CHAIN_FP64
+#error "compile with -DQND_CHAIN_FP64=0 or 1"
+#endif
+
+namespace qnd {
+
+// Sums of n (at most MAX_RED) accumulators over the CTA's T threads, to out[0..n) in shared memory,
+// visible to every thread on return. red: [T / 32][MAX_RED] shared scratch.
+template <int T> __device__ __forceinline__ void cta_sums(const double* acc, int n, double (*red)[MAX_RED], double* out) {
+    const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
+#pragma unroll
+    for (int k = 0; k < MAX_RED; ++k) {
+        if (k >= n) break;
+        const double s = warp_sum(acc[k]);
+        if (lane == 0) red[wid][k] = s;
+    }
+    __syncthreads();
+    if (t < n) {
+        double s = 0.0;
+        for (int w = 0; w < T / 32; ++w) s += red[w][t];
+        out[t] = s;
+    }
+    __syncthreads();
+}
+
+// Threads per line and the shared memory of a chain: E values per thread.
+template <typename R, int L, int E> struct ChainShape {
+    using P = FFTPlan<L, E>;
+    static constexpr int T = L / E;
+    static constexpr int TW = ((sizeof(R) == 8 ? P::twb_size() : P::tw_size()) + 1) & ~1;
+    static constexpr size_t SMEM = sizeof(cplx_t<R>) * (size_t(TW) + P::SMEM_LINE);
+};
+
+template <typename R, int L, int E>
+__global__ void __launch_bounds__(L / E, 1) qnd_chain1d_kernel(const __grid_constant__ Chain1dArgs<R> a) {
+    using V = cplx_t<R>;
+    using SH = ChainShape<R, L, E>;
+    constexpr int T = SH::T;
+    static_assert(T >= 32 && T % 32 == 0, "whole warps");
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    __shared__ double red_s[T / 32][MAX_RED];
+    __shared__ double sum_s[MAX_RED];
+    __shared__ double coef_s[2 * GS_MAXK];
+    V* tw = reinterpret_cast<V*>(smem_raw);
+    V* line = tw + SH::TW;
+    const int tid = threadIdx.x;
+    const LineSync<T> lsync{1};
+    const int shift1 = 0;
+    const long long nmask1 = L - 1;
+
+    for (int i = tid; i < (sizeof(R) == 8 ? SH::P::twb_size() : SH::P::tw_size()); i += T) tw[i] = a.tw[i];
+    V v[E];
+#pragma unroll
+    for (int u = 0; u < E; ++u) v[u] = a.psi[tid + u * T];
+    __syncthreads();  // twiddles visible
+
+    // the point-wise factor `mid` (a full-grid table) with the laser phases at `laser`, the step mask
+    // and a device scalar
+    auto factors = [&](int mid, int laser, bool mask, const double* scale, uint32_t key) {
+        const V* axc[1] = {laser >= 0 ? a.field + laser : nullptr};
+        const R* axr[1] = {mask ? a.mask : nullptr};
+        apply_factors<R, E, T>(v, tid, 0, 0, mid >= 0 ? a.mid_real[mid] : nullptr, mid >= 0 ? a.mid_cplx[mid] : nullptr,
+                               axc, axr, 0, 1, &shift1, &nmask1, scale, key);
+    };
+    factors(a.pre_mid, a.pre_laser, false, a.pre_scale, mix32(a.seed) ^ 0x51ed270bu);
+
+#pragma unroll 1
+    for (int i = 0; i < a.nops; ++i) {
+        const Chain1dOp op = a.ops[i];
+        const uint32_t key = mix32(a.seed + 0x9e3779b9u * uint32_t(i + 1));
+        const V* __restrict__ sp = op.spec >= 0 ? a.spec[op.spec] : a.field + op.field_spec;
+        V f[E];  // the spectral row, on its way during the forward transform
+#pragma unroll
+        for (int u = 0; u < E; ++u) f[u] = __ldg(sp + tid + u * T);
+        fft_line_stages<L, E, -1, 0, true>(v, tid, line, tw, lsync);
+#pragma unroll
+        for (int u = 0; u < E; ++u)
+            v[u] = fmul_spec<L>(v[u], f[u], key + uint32_t(tid + u * T), u == 0 || u == E - 1);
+        fft_line_stages<L, E, +1, 0, true>(v, tid, line, tw, lsync);
+        factors(op.mid, op.laser, op.mask != 0, nullptr, key ^ 0x2545f491u);
+        if (op.obs >= 0) {
+            double acc[MAX_RED];
+#pragma unroll
+            for (int k = 0; k < MAX_RED; ++k) acc[k] = 0.0;
+            accumulate_line<R, E, T>(a.red, acc, v, static_cast<const V*>(nullptr), 0, 0, 0, tid, 0, &shift1, &nmask1);
+            cta_sums<T>(acc, a.red.n, red_s, sum_s);
+            if (tid < a.red.n) a.red.out[op.obs + tid] = sum_s[tid] * a.red.scale[tid];
+        }
+        if (op.gs) {
+            // v = psi - sum_k <psi_k|psi> psi_k, then v / ||v|| (QuantumND_imag.c:280-310)
+            for (int k0 = 0; k0 < a.ngs; k0 += MAX_RED / 2) {
+                double acc[MAX_RED];
+#pragma unroll
+                for (int q = 0; q < MAX_RED / 2; ++q) {
+                    acc[2 * q] = acc[2 * q + 1] = 0.0;
+                    if (k0 + q >= a.ngs) continue;
+                    const V* __restrict__ s = a.states[k0 + q];
+#pragma unroll
+                    for (int u = 0; u < E; ++u) {
+                        const V p = s[tid + u * T];
+                        acc[2 * q] += double(p.x) * double(v[u].x) + double(p.y) * double(v[u].y);
+                        acc[2 * q + 1] += double(p.x) * double(v[u].y) - double(p.y) * double(v[u].x);
+                    }
+                }
+                const int n = 2 * (a.ngs - k0 < MAX_RED / 2 ? a.ngs - k0 : MAX_RED / 2);
+                cta_sums<T>(acc, n, red_s, sum_s);
+                if (tid < n) coef_s[2 * k0 + tid] = sum_s[tid] * a.dNr;
+                __syncthreads();
+            }
+            for (int k = 0; k < a.ngs; ++k) {
+                const V* __restrict__ s = a.states[k];
+                const R cr = R(coef_s[2 * k]), ci = R(coef_s[2 * k + 1]);
+#pragma unroll
+                for (int u = 0; u < E; ++u) {
+                    const V p = s[tid + u * T];
+                    v[u].x -= cr * p.x - ci * p.y;
+                    v[u].y -= cr * p.y + ci * p.x;
+                }
+            }
+            double acc[1] = {0.0};
+#pragma unroll
+            for (int u = 0; u < E; ++u) acc[0] += double(v[u].x) * double(v[u].x) + double(v[u].y) * double(v[u].y);
+            cta_sums<T>(acc, 1, red_s, sum_s);
+            const double n2 = sum_s[0] * a.dNr;
+            double scale = 1.0;
+            if (n2 < a.gs_tol || !(n2 == n2)) {
+                if (tid == 0) *a.gs_flag = 1;
+            } else {
+                scale = 1.0 / sqrt(n2);
+            }
+            const R sc = R(scale);
+#pragma unroll
+            for (int u = 0; u < E; ++u) v[u] = cscale(v[u], sc);
+        }
+        if (op.mid2 >= 0) factors(op.mid2, -1, false, nullptr, key ^ 0x68e31da4u);
+    }
+#pragma unroll
+    for (int u = 0; u < E; ++u) a.psi[tid + u * T] = v[u];
+}
+
+template <typename R, int L> static cudaError_t launch_one(const Chain1dArgs<R>& a, cudaStream_t st) {
+    constexpr int E = chain1d_values(L);
+    using SH = ChainShape<R, L, E>;
+    auto* fn = &qnd_chain1d_kernel<R, L, E>;
+    if constexpr (SH::SMEM > 48 * 1024) {
+        const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(SH::SMEM));
+        if (e != cudaSuccess) return e;
+    }
+    fn<<<1, SH::T, SH::SMEM, st>>>(a);
+    return cudaGetLastError();
+}
+
+template <typename R> cudaError_t launch_chain1d(int L, const Chain1dArgs<R>& a, cudaStream_t st) {
+    switch (L) {
+    case 128: return launch_one<R, 128>(a, st);
+    case 256: return launch_one<R, 256>(a, st);
+    case 512: return launch_one<R, 512>(a, st);
+    case 1024: return launch_one<R, 1024>(a, st);
+    case 2048: return launch_one<R, 2048>(a, st);
+    case 4096: return launch_one<R, 4096>(a, st);
+    default: return cudaErrorInvalidValue;
+    }
+}
+
+#if QND_CHAIN_FP64
+template cudaError_t launch_chain1d<double>(int, const Chain1dArgs<double>&, cudaStream_t);
+#else
+template cudaError_t launch_chain1d<float>(int, const Chain1dArgs<float>&, cudaStream_t);
+#endif
+
+}  // namespace qnd

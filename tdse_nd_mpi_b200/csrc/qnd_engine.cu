@@ -167,6 +167,7 @@ struct qnd_ctx {
     uint64_t table_epoch = 0;  // bumps when V / Vcap change; invalidates r-space tables
 
     DevBuf tw[MAX_DIM];
+    DevBuf tw_chain;      // 1-D grids the chain kernel takes: its stage twiddles (run_chain1d)
     DevBuf r_dev, p_dev;  // concatenated axes (double)
     DevBuf gradv_dev[MAX_DIM];                // natural layout
     DevBuf gradv_lm[MAX_DIM][MAX_DIM];        // [component][pass axis] line-major copies
@@ -297,9 +298,9 @@ static void round_pairs_f32_balanced(const double* v, size_t n, float* out) {
     }
 }
 
-// Stage twiddles of HostPlan(L) (for E values per thread, default the pass kernels'), exp(-2 pi i jm r / (Ns R)) in long double: FP64 plans one base per
-// butterfly position (r = 1; the kernel forms the powers, TwiddledDFT), FP32 plans every r in the
-// [j mod Ns][r-1] layout.
+// Stage twiddles of HostPlan(L) (for E values per thread, default the pass kernels'), exp(-2 pi i jm r /
+// (Ns R)) in long double: FP64 plans one base per butterfly position (r = 1; the kernel forms the
+// powers, TwiddledDFT), FP32 plans every r in the [j mod Ns][r-1] layout.
 static void build_twiddles(qnd_ctx* c, int L, DevBuf& dst, int E = 0) {
     HostPlan pl(L, E ? E : lookup_pass(c->fp64, L, false, PM_SANDWICH).E);
     const int entries = c->fp64 ? pl.twb_size : pl.tw_size;
@@ -915,6 +916,27 @@ static int shape_choice(qnd_ctx* c, const PassSpec& ps, int L, int log2S, int km
 
 static void emulate_long_pass(qnd_ctx* c, const PassSpec& ps);
 
+// While profiling, events around a pass launch (qnd_ctx_set_profiling).
+static std::pair<cudaEvent_t, cudaEvent_t> profile_begin(qnd_ctx* c) {
+    std::pair<cudaEvent_t, cudaEvent_t> ev{nullptr, nullptr};
+    if (!c->profiling) return ev;
+    for (cudaEvent_t* e : {&ev.first, &ev.second}) {
+        if (c->event_pool.empty()) {
+            QND_CK(cudaEventCreate(e));
+        } else {
+            *e = c->event_pool.back();
+            c->event_pool.pop_back();
+        }
+    }
+    QND_CK(cudaEventRecord(ev.first, c->stream));
+    return ev;
+}
+static void profile_end(qnd_ctx* c, const std::pair<cudaEvent_t, cudaEvent_t>& ev) {
+    if (!ev.first) return;
+    QND_CK(cudaEventRecord(ev.second, c->stream));
+    c->prof_pairs.push_back(ev);
+}
+
 // Launch one fused axis pass: persistent grid (at most the resident CTAs), programmatic
 // dependent launch so the pass's prologue overlaps the tail of the previous kernel.
 static void launch_pass(qnd_ctx* c, const PassSpec& ps) {
@@ -1013,18 +1035,7 @@ static void launch_pass(qnd_ctx* c, const PassSpec& ps) {
         red.partials = c->partials.as<double>();
         red.counter = c->counter.as<unsigned int>();
     }
-    std::pair<cudaEvent_t, cudaEvent_t> ev{nullptr, nullptr};
-    if (c->profiling) {
-        for (cudaEvent_t* e : {&ev.first, &ev.second}) {
-            if (c->event_pool.empty()) {
-                QND_CK(cudaEventCreate(e));
-            } else {
-                *e = c->event_pool.back();
-                c->event_pool.pop_back();
-            }
-        }
-        QND_CK(cudaEventRecord(ev.first, c->stream));
-    }
+    const auto ev = profile_begin(c);
     cudaLaunchConfig_t lc{};
     lc.gridDim = dim3(unsigned(blocks));
     lc.blockDim = dim3(unsigned(kinfo.nt));
@@ -1061,10 +1072,7 @@ static void launch_pass(qnd_ctx* c, const PassSpec& ps) {
         QND_CK(cudaLaunchKernelExC(&lc, kinfo.fn, args));
     }
     c->kernels_launched++;
-    if (c->profiling) {
-        QND_CK(cudaEventRecord(ev.second, c->stream));
-        c->prof_pairs.push_back(ev);
-    }
+    profile_end(c, ev);
 }
 
 static int reduce_blocks(qnd_ctx* c) {
@@ -1705,7 +1713,10 @@ struct ChainMid {
     int64_t lst = 0;
     bool mask = false;
     const RedDesc* red = nullptr;
-    bool empty() const { return f.kind < 0 && f.laser_ia < 0 && !mask && !red; }
+    // chain kernel only (1-D): Gram-Schmidt against the states run_chain1d is given, then a second factor
+    bool gs = false;
+    Factor f2;
+    bool empty() const { return f.kind < 0 && f.laser_ia < 0 && !mask && !red && !gs && f2.kind < 0; }
 };
 
 static void set_factor(qnd_ctx* c, const Factor& f, int ax, int64_t lst, const void** treal, const void** tcplx,
@@ -1733,6 +1744,105 @@ static int sandwich_last_axis(const qnd_ctx* c, int64_t i) {
 // Axis of the chain's last pass (the one that carries the final factor, mask and reductions).
 static int chain_final_axis(const qnd_ctx* c, int NK) { return sandwich_last_axis(c, NK - 1); }
 
+// 1-D grids whose chains run in one launch of the chain kernel (qnd_chain1d.cu): lengths of 128 to 4096
+// points. A pass of such a grid is one CTA on one SM, so a launch per pair of sandwiches left the GPU
+// waiting on launches and on the state's round trip: a BM4 step took 77 us at 4096 points (with
+// Gram-Schmidt) and 34 us at 512 (with observables) by passes, and takes 37 and 12.7 us by this kernel. Shorter lines have fewer than a warp of
+// 4-point threads and keep the passes, as do the recorded passes of the persistent sweep kernel.
+static bool chain1d(const qnd_ctx* c) { return c->tw_chain.p && !c->recorder; }
+
+struct ChainGs {
+    void* const* states = nullptr;  // the earlier states
+    int n = 0;
+};
+
+static void run_chain1d(qnd_ctx* c, void* psi, const std::vector<ChainK>& K, const std::vector<ChainMid>& M,
+                        const Factor& pre, int64_t pre_lst, const double* pre_scale, const ChainMid& post,
+                        const ChainGs& gs = ChainGs()) {
+    const int64_t NK = int64_t(K.size());
+    auto run = [&](auto tag) {
+        using R = decltype(tag);
+        using V = cplx_t<R>;
+        auto ap = std::make_unique<Chain1dArgs<R>>();
+        Chain1dArgs<R>& a = *ap;
+        const V* field = static_cast<const V*>(c->field_view ? c->field_view : c->field_tab.p);
+        std::vector<ChainK> specs;     // distinct tables of the launch being filled
+        std::vector<Factor> mids;
+        auto begin = [&]() {
+            a = Chain1dArgs<R>{};
+            a.psi = static_cast<V*>(psi);
+            a.tw = c->tw_chain.as<V>();
+            a.field = field;
+            a.mask = c->mask_dev[0].as<R>();
+            a.pre_mid = a.pre_laser = -1;
+            a.dNr = c->dNr;
+            a.gs_tol = 1.e-12;
+            a.gs_flag = c->gs_flag.as<int>();
+            a.ngs = gs.n;
+            for (int k = 0; k < gs.n; ++k) a.states[k] = static_cast<const V*>(gs.states[k]);
+            specs.clear();
+            mids.clear();
+        };
+        auto laser_at = [&](int64_t lst, int ia) {
+            return int((static_cast<const char*>(field_slice(c, lst, ia, 0)) - reinterpret_cast<const char*>(field)) /
+                       int64_t(sizeof(V)));
+        };
+        auto spec_id = [&](const ChainK& k) {
+            for (size_t q = 0; q < specs.size(); ++q)
+                if (specs[q].kind == k.kind && specs[q].coef == k.coef) return short(q);
+            a.spec[specs.size()] = static_cast<const V*>(spec_table(c, k.kind, 0, k.coef));
+            specs.push_back(k);
+            return short(specs.size() - 1);
+        };
+        auto mid_id = [&](const Factor& f) {
+            if (f.kind < 0) return short(-1);
+            for (size_t q = 0; q < mids.size(); ++q)
+                if (mids[q].kind == f.kind && mids[q].a == f.a && mids[q].b == f.b) return short(q);
+            const void* t = rtab(c, f.kind, f.a, f.b);
+            if (f.kind == RT_IMAG) a.mid_real[mids.size()] = static_cast<const R*>(t);
+            else a.mid_cplx[mids.size()] = static_cast<const V*>(t);
+            mids.push_back(f);
+            return short(mids.size() - 1);
+        };
+        auto launch = [&]() {
+            a.seed = uint32_t(c->kernels_launched) * 0x9e3779b9u + 0x632be5abu;
+            const auto ev = profile_begin(c);
+            QND_CK(launch_chain1d<R>(int(c->nr[0]), a, c->stream));
+            c->kernels_launched++;
+            profile_end(c, ev);
+        };
+        begin();
+        a.pre_mid = mid_id(pre);
+        if (pre.laser_ia >= 0) a.pre_laser = laser_at(pre_lst, pre.laser_ia);
+        a.pre_scale = pre_scale;
+        for (int64_t i = 0; i < NK; ++i) {
+            if (a.nops == CHAIN1D_OPS || specs.size() + 1 > CHAIN1D_TABLES || mids.size() + 2 > CHAIN1D_TABLES) {
+                launch();
+                begin();
+            }
+            const ChainMid& m = i + 1 < NK ? M[i] : post;
+            Chain1dOp& op = a.ops[a.nops++];
+            if (K[i].kind == KV_FIELD) op.field_spec = laser_at(K[i].lst, K[i].ia);
+            else op.spec = spec_id(K[i]);
+            op.mid = mid_id(m.f);
+            if (m.f.laser_ia >= 0) op.laser = laser_at(m.lst, m.f.laser_ia);
+            op.mask = m.mask && a.mask;
+            if (m.red) {
+                if (!a.red.n) {
+                    a.red = *m.red;
+                    set_red_axes(c, a.red);
+                }
+                op.obs = int(m.red->out - a.red.out);
+            }
+            op.gs = m.gs;
+            op.mid2 = mid_id(m.f2);
+        }
+        launch();
+    };
+    if (c->fp64) run(double{});
+    else run(float{});
+}
+
 // Run a chain of kinetic sandwiches K_0 .. K_{NK-1} with M[i] between K_i and K_{i+1}, `pre` (and
 // the device scalar pre_scale) before K_0 and `post` after K_{NK-1}. Consecutive sandwiches run
 // their axes in opposite orders, so the last axis of K_i is the first axis of K_{i+1}: those two
@@ -1745,6 +1855,10 @@ static void run_chain(qnd_ctx* c, void* psi, const std::vector<ChainK>& K, const
     const int d = c->dim;
     const int64_t NK = int64_t(K.size());
     if (NK == 0 || int64_t(M.size()) != NK - 1) QND_FAIL(QND_EINVAL, "internal: malformed sandwich chain");
+    if (chain1d(c)) {
+        run_chain1d(c, psi, K, M, pre, pre_lst, pre_scale, post);
+        return;
+    }
     if (c->long1d) {
         // four-step sandwiches: length-n1 forward, the length-n2 sandwich pass (twiddles, slot-order
         // k-space table, conjugate twiddles), then either one length-n1 roundtrip pass (inverse,
@@ -1891,13 +2005,46 @@ static void imag_steps(qnd_ctx* c, void* psi, int64_t nsteps, const double* pro_
     run_chain(c, psi, K, M, pre, 0, pro_scale, post);
 }
 
+// n x {imaginary-time step, Gram-Schmidt against gs.states, normalisation} on a grid of the chain kernel.
+static void imag_chain1d(qnd_ctx* c, void* psi, int64_t n, const ChainGs& gs) {
+    const int s = c->s;
+    std::vector<ChainK> K;
+    std::vector<ChainMid> M;
+    for (int64_t st = 0; st < n; ++st)
+        for (int i = 0; i < s; ++i) {
+            ChainK k;
+            k.kind = SP_IMAG;
+            k.coef = c->as[2 * i] + c->as[2 * i + 1];
+            K.push_back(k);
+            ChainMid m;
+            m.f.kind = RT_IMAG;
+            m.f.a = c->as[2 * i + 1];
+            if (i + 1 < s) {
+                m.f.b = c->as[2 * i + 2];
+            } else {
+                m.gs = true;
+                if (st + 1 < n) {
+                    m.f2.kind = RT_IMAG;
+                    m.f2.a = c->as[0];
+                }
+            }
+            M.push_back(m);
+        }
+    const ChainMid post = M.back();
+    M.pop_back();
+    Factor pre;
+    pre.kind = RT_IMAG;
+    pre.a = c->as[0];
+    run_chain1d(c, psi, K, M, pre, 0, nullptr, post, gs);
+}
+
 // Length-gauge steps lst0 .. lst0+n-1 of the current field chunk in r-space (integrators.c:170-194
 // rewritten in r-space): per step K(a_0) V(h_0) K(a_1 + a_2) V(h_1) ... V(h_{s-1}) K(a_{2s-1}); after
 // each step the step mask and the reductions red_fn(k, .) (of psi(t_{k+1})). A step boundary with
 // nothing on it merges K(a_{2s-1}) with the next step's K(a_0).
 static void length_steps(qnd_ctx* c, void* psi, int64_t lst0, int64_t n, const RedFn& red_fn, bool masked) {
     if (n <= 0) return;
-    if (c->dim == 1 && !c->long1d && n > 1 && (masked || red_fn)) {
+    if (c->dim == 1 && !c->long1d && !chain1d(c) && n > 1 && (masked || red_fn)) {
         // 1-D chains carry boundary work only at their end
         for (int64_t k = 0; k < n; ++k)
             length_steps(c, psi, lst0 + k, 1, red_fn ? RedFn([&](int64_t, int ax) { return red_fn(k, ax); }) : RedFn(),
@@ -1956,10 +2103,19 @@ static void length_steps(qnd_ctx* c, void* psi, int64_t lst0, int64_t n, const R
 
 // Velocity-gauge steps lst0 .. lst0+n-1 in r-space (integrators.c:201-232); between steps the
 // factors V(a_{2s-1}) V(a_0) merge into one. The step mask and the reductions `fin` apply after the
-// last step only.
-static void velocity_steps(qnd_ctx* c, void* psi, int64_t lst0, int64_t n, const RedDesc* fin, bool masked) {
+// last step only; on the grids of the chain kernel (chain1d), red_fn (in place of fin) and the mask
+// apply after every step.
+static void velocity_steps(qnd_ctx* c, void* psi, int64_t lst0, int64_t n, const RedDesc* fin, bool masked,
+                           const RedFn& red_fn = RedFn()) {
     if (n <= 0) return;
     const int s = c->s;
+    std::vector<std::vector<RedDesc>> reds;
+    reds.reserve(size_t(n));
+    auto reductions = [&](int64_t k) -> const RedDesc* {
+        if (!red_fn) return nullptr;
+        reds.push_back(red_fn(k, 0));
+        return reds.back().empty() ? nullptr : &reds.back()[0];
+    };
     std::vector<ChainK> K;
     std::vector<ChainMid> M;
     for (int64_t k = 0; k < n; ++k)
@@ -1969,6 +2125,15 @@ static void velocity_steps(qnd_ctx* c, void* psi, int64_t lst0, int64_t n, const
                 m.f.kind = RT_VEL;
                 m.f.a = i > 0 ? c->as[2 * i - 1] : c->as[2 * s - 1];
                 m.f.b = c->as[2 * i];
+                if (i == 0 && chain1d(c)) {
+                    m.red = reductions(k - 1);
+                    m.mask = masked;
+                    if (m.red || m.mask) {  // something between the two factors of the step boundary
+                        m.f.b = NO_COEF;
+                        m.f2.kind = RT_VEL;
+                        m.f2.a = c->as[0];
+                    }
+                }
                 M.push_back(m);
             }
             ChainK kk;
@@ -1984,7 +2149,7 @@ static void velocity_steps(qnd_ctx* c, void* psi, int64_t lst0, int64_t n, const
     post.f.a = c->as[2 * s - 1];
     post.lst = lst0 + n - 1;
     post.mask = masked;
-    post.red = fin;
+    post.red = red_fn ? reductions(n - 1) : fin;
     run_chain(c, psi, K, M, pre, lst0, nullptr, post);
 }
 
@@ -2101,10 +2266,10 @@ static void run_chunk_graph(qnd_ctx* c, const std::string& key, const std::funct
     QND_CK(cudaGraphLaunch(ex, c->stream));
 }
 
-// What a length-gauge chunk chain captures (see run_chunk_graph).
+// What a chunk chain of either gauge captures (see run_chunk_graph).
 static std::string chain_key(qnd_ctx* c, const void* psi, int64_t ch, int nobs, const char* const* names,
-                             const double* rows, bool masked) {
-    std::string k = fmt("L|%llu|%p|%lld|%p|%d|%p|%p|%p|%llu|%llu|%d|", (unsigned long long)c->serial, psi,
+                             const double* rows, bool masked, bool velocity = false) {
+    std::string k = fmt("%c|%llu|%p|%lld|%p|%d|%p|%p|%p|%llu|%llu|%d|", velocity ? 'V' : 'L', (unsigned long long)c->serial, psi,
                         (long long)ch, (const void*)rows, int(masked), c->field_tab.p, c->partials.p, c->counter.p,
                         (unsigned long long)c->table_epoch, (unsigned long long)c->config_epoch, int(c->pdl));
     for (int q = 0; q < nobs; ++q) {
@@ -2129,8 +2294,10 @@ static void run_realtime(qnd_ctx* c, void* psi, const double* field_host, const 
     }
     std::vector<double> zero_alpha(MAX_DIM, 0.0);
     double* rows = c->obs_dev.as<double>();
-    // length gauge whose observables are r-space reductions of one descriptor: chunk-wide chains
-    const bool chain = !velocity && (nv == 0 || (fused && rspace_red(c, items, rows, 0).size() <= 1));
+    // observables that are r-space reductions of one descriptor: chunk-wide chains (velocity gauge: on
+    // the grids of the chain kernel)
+    const bool chain = (velocity ? chain1d(c) : true) &&
+                       (nv == 0 || (all_rspace(items) && rspace_red(c, items, rows, 0).size() <= 1));
     for (int64_t c0 = 0; c0 < nsteps; c0 += ch_max) {
         const int64_t ch = std::min(ch_max, nsteps - c0);
         if (nv > 0 && c0 == 0) {
@@ -2143,8 +2310,10 @@ static void run_realtime(qnd_ctx* c, void* psi, const double* field_host, const 
             // pass that straddles the step boundary
             RedFn rf;
             if (nv > 0) rf = [&](int64_t k, int ax) { return rspace_red(c, items, rows + size_t(k + 1) * nv, ax); };
-            run_chunk_graph(c, chain_key(c, psi, ch, nobs, names, rows, masked),
-                            [&]() { length_steps(c, psi, 0, ch, rf, masked); });
+            run_chunk_graph(c, chain_key(c, psi, ch, nobs, names, rows, masked, velocity), [&]() {
+                if (velocity) velocity_steps(c, psi, 0, ch, nullptr, masked, rf);
+                else length_steps(c, psi, 0, ch, rf, masked);
+            });
         } else {
             for (int64_t k = 0; k < ch; ++k) {
                 const int64_t gst = c0 + k;
@@ -2435,16 +2604,21 @@ static void adjoint_run(qnd_ctx* c, const void* psi0, const double* F, int64_t n
 
 // ---------------------------------------------------------------- Gram-Schmidt --
 
-// v = psi_j - sum_k <psi_k|psi_j> psi_k; norm2 = ||v||^2 dNr into scal[0]; scale 1/sqrt(norm2) into
-// scal[1]; the flag is raised when norm2 < 1e-12 (QuantumND_imag.c:280-304). The normalisation itself
-// is left to the caller (scale kernel or the next step's prologue).
-static void gs_project(qnd_ctx* c, void* const* states, int j) {
+// The scalars and the norm-collapse flag of Gram-Schmidt against j states.
+static void prepare_gs(qnd_ctx* c, int j) {
     if (j >= GS_MAXK) QND_FAIL(QND_EUNSUPPORTED, "Gram-Schmidt against %d states (max %d)", j, GS_MAXK - 1);
     c->scal.ensure(sizeof(double) * (2 + 2 * GS_MAXK));
     if (!c->gs_flag.p) {
         c->gs_flag.ensure(sizeof(int));
         QND_CK(cudaMemsetAsync(c->gs_flag.p, 0, sizeof(int), c->stream));
     }
+}
+
+// v = psi_j - sum_k <psi_k|psi_j> psi_k; norm2 = ||v||^2 dNr into scal[0]; scale 1/sqrt(norm2) into
+// scal[1]; the flag is raised when norm2 < 1e-12 (QuantumND_imag.c:280-304). The normalisation itself
+// is left to the caller (scale kernel or the next step's prologue).
+static void gs_project(qnd_ctx* c, void* const* states, int j) {
+    prepare_gs(c, j);
     double* scal = c->scal.as<double>();
     const int nb = reduce_blocks(c);
     ensure_red_scratch(c, nb);
@@ -2658,6 +2832,7 @@ static void build_context(qnd_ctx* c, int dim, const int64_t* nr, const double* 
             build_twiddles(c, int(c->nr[j]), c->tw[j]);
         }
     }
+    if (dim == 1 && chain1d_length_ok(c->nr[0])) build_twiddles(c, int(c->nr[0]), c->tw_chain, chain1d_values(int(c->nr[0])));
     if (any_long) {
         // the scratch states of the emulated passes, allocated up front (not inside a graph capture)
         c->lax_perm.ensure(size_t(c->n) * c->elem());
@@ -3086,6 +3261,20 @@ int qnd_imag_propagate(qnd_ctx* ctx, void* const* states_dev, int j, int64_t nst
     for (int k = 0; k <= j; ++k) QND_NEED(states_dev[k]);
     if (nsteps <= 0) return QND_OK;
     set_device(ctx);
+    if (chain1d(ctx)) {
+        // the chain kernel does the steps, Gram-Schmidt and the normalisation of a block in one go
+        check_imag_clamp(ctx);
+        prepare_gs(ctx, j);
+        ChainGs gs;
+        gs.states = states_dev;
+        gs.n = j;
+        for (int64_t st = 0; st < nsteps; st += CHUNK) {
+            imag_chain1d(ctx, states_dev[j], std::min(CHUNK, nsteps - st), gs);
+            check_gs_flag(ctx, j);
+        }
+        check_finite(ctx, states_dev[j], "qnd_imag_propagate");
+        return QND_OK;
+    }
     // the first step, then blocks of up to CHUNK steps {step with the deferred normalisation,
     // Gram-Schmidt}, each replayed from a CUDA graph once its shape has been seen (run_chunk_graph);
     // the norm-collapse flag is read after every block

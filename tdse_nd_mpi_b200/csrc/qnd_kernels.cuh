@@ -201,6 +201,46 @@ template <typename R> void launch_axis_permute(const AxisPermArgs& a, const cplx
 template <typename R> void launch_apply_combine(long long n, cplx_t<R>* dst, const cplx_t<R>* tmp,
                                                const cplx_t<R>* src, const double* vtab, int acc, cudaStream_t st);
 
+// ---- 1-D grids of up to 4096 points: a chain of sandwiches in one launch (qnd_chain1d.cu)
+constexpr int CHAIN1D_OPS = 512;     // sandwiches per launch (longer chains take several launches)
+constexpr int CHAIN1D_TABLES = 24;   // distinct spectral / r-space tables per launch
+// Line lengths the chain kernel is built for, and its values per thread (whole warps on one line).
+// Measured with FP64, us per BM4 step with observables: 512 points 12.7 with 8 values (4: 16.6, 16: 19.1),
+// 1024 19.1 (16: 21.4), 2048 27.7 with 16 (8: 29.6), 4096 (imaginary time) 37 with 16 (8: 44).
+constexpr bool chain1d_length_ok(long long L) { return L >= 128 && L <= 4096 && (L & (L - 1)) == 0; }
+constexpr int chain1d_values(int L) { return L == 128 ? 4 : (L < 2048 ? 8 : 16); }
+// One sandwich and the point-wise work after it, in this order: factor `mid` with the laser phases and
+// the step mask, reductions into red.out + obs, Gram-Schmidt, factor `mid2`.
+struct Chain1dOp {
+    short spec = -1;      // spectral table, -1: the field-table row at field_spec
+    short mid = -1, mid2 = -1;
+    unsigned char mask = 0, gs = 0;
+    int field_spec = 0;
+    int laser = -1;       // field-table offset of the laser phases
+    int obs = -1;
+};
+template <typename R> struct Chain1dArgs {
+    using V = cplx_t<R>;
+    V* psi;
+    const V* tw;          // stage twiddles for chain1d_values(L) values per thread
+    const V* field;       // per-step field tables
+    const V* spec[CHAIN1D_TABLES];
+    const R* mid_real[CHAIN1D_TABLES];
+    const V* mid_cplx[CHAIN1D_TABLES];
+    const R* mask;
+    int pre_mid, pre_laser;       // before the first sandwich (-1: none), with *pre_scale (may be null)
+    const double* pre_scale;
+    unsigned seed;
+    RedDesc red;                  // out: the row that obs = 0 names
+    const V* states[GS_MAXK];     // Gram-Schmidt: the earlier states
+    int ngs;
+    int* gs_flag;
+    double dNr, gs_tol;
+    int nops;
+    Chain1dOp ops[CHAIN1D_OPS];
+};
+template <typename R> cudaError_t launch_chain1d(int L, const Chain1dArgs<R>& a, cudaStream_t st);
+
 // ---- the persistent sweep kernel (qnd_sweep.cu): recorded passes of many members in one launch
 constexpr int SWEEP_NT = 128;  // threads per CTA: every line length it takes has 128-thread pass CTAs
 // One recorded pass of one member: its arguments (PassArgs<R> in device memory), its line groups,

@@ -23,9 +23,10 @@
 //   PM_SPECRED   reductions of |FFT psi|^2 weighted by k-space tables; no write
 //   PM_APPLY     u = IFFT[spec . FFT psi] (+ V psi) (+ dst); optional store into dst and
 //                reductions of |u|^2 or Re(conj(partner) u)   (energy moments, Lz)
-//   PM_ROUNDTRIP psi <- FFT[ mid(x) . scale . IFFT[psi] ]: the closing inverse transform of one
-//                sandwich and the opening transform of the next on the strided virtual axis of a
-//                long 1-D axis, with the r-space factors between (tables in natural order)
+//   PM_ROUNDTRIP psi <- FFT[ mid(x) . scale . IFFT[psi] ] (+ reductions before the FFT): the closing
+//                inverse transform of one sandwich and the opening transform of the next on the
+//                strided virtual axis of a long 1-D axis, with the r-space factors between. Every table,
+//                those of the axis itself among them, is in the line-major order of this axis.
 //
 // Reductions are FP64 and deterministic: per-CTA partial sums, then the last CTA
 // to finish (ticket counter) adds the partials in a fixed order.
@@ -51,15 +52,18 @@ enum : int {
     PM_SANDWICH_RED = 7,  // PM_SANDWICH / PM_DOUBLE with fused reductions: separate instantiations, so that
     PM_DOUBLE_RED = 8,    // the passes without reductions (most of a chain) keep their registers for the FFT;
     PM_DOUBLE_RED_END = 9,  // PM_DOUBLE_RED reduces between its sandwiches (a step boundary), _END after both
-    PM_NMODES = 10
+    PM_ROUNDTRIP_RED = 10,
+    PM_NMODES = 11
 };
 // The transform structure of a mode (the reducing variants share their base mode's) and whether the
 // mode can carry reductions at all.
 __host__ __device__ constexpr int pass_base_mode(int m) {
-    return m == PM_SANDWICH_RED ? PM_SANDWICH : ((m == PM_DOUBLE_RED || m == PM_DOUBLE_RED_END) ? PM_DOUBLE : m);
+    return m == PM_SANDWICH_RED ? PM_SANDWICH
+           : (m == PM_DOUBLE_RED || m == PM_DOUBLE_RED_END) ? PM_DOUBLE
+           : m == PM_ROUNDTRIP_RED ? PM_ROUNDTRIP : m;
 }
 __host__ __device__ constexpr bool pass_mode_reduces(int m) {
-    return m == PM_SANDWICH_RED || m == PM_DOUBLE_RED || m == PM_DOUBLE_RED_END || m == PM_SPECRED || m == PM_APPLY;
+    return m == PM_SANDWICH_RED || m == PM_ROUNDTRIP_RED || m == PM_DOUBLE_RED || m == PM_DOUBLE_RED_END || m == PM_SPECRED || m == PM_APPLY;
 }
 // |v|^2 w, Re(conj(partner) v) w, or (element-wise grid reductions only) Im(conj(partner) v) w and
 // the count of elements with a non-finite part
@@ -430,15 +434,14 @@ template <int NT> __device__ __forceinline__ void finish_red(const RedDesc& rd, 
 // Point-wise r-space factors on the E values a thread holds of one line: a full-grid table
 // (line-major: entry lbase + m), per-axis complex factors (the pass axis per element, the other
 // axes once per line), per-axis real factors and a scalar.
-// NAT: every table is indexed by the element's natural point index base + (m << log2S) instead of
-// the line-major lbase + m and the position m along the pass axis (the strided virtual axis of a
-// long 1-D axis, whose tables are in natural order).
-template <typename R, int E, int T, bool NAT = false>
+// ROWS: the per-axis tables are rows of full tables in line-major order (entry lbase + m) too, not
+// tables over the position m (the strided virtual axis of a long 1-D axis).
+template <typename R, int E, int T, bool ROWS = false>
 __device__ __forceinline__ void apply_factors(cplx_t<R>* v, int tid, long long base, long long lbase,
                                               const R* __restrict__ tr, const cplx_t<R>* __restrict__ tc,
                                               const cplx_t<R>* const* axc, const R* const* axr, int axis, int dim,
                                               const int* shift, const long long* nmask, const double* scale_dev,
-                                              uint32_t key, int log2S = 0) {
+                                              uint32_t key) {
     using V = cplx_t<R>;
     V lf = fone<V>();
     R lr = R(1);
@@ -465,11 +468,8 @@ __device__ __forceinline__ void apply_factors(cplx_t<R>* v, int tid, long long b
     // every read waited for the one before it, and the factor between the sandwiches of a 1024-point
     // two-sandwich pass took 16,500 of the pass's 55,000 cycles (FP64; 8,000 to 9,600 of 37,000 in
     // FP32). The order of an element's products is the same.
-    auto grid_at = [&](int u) {  // full-grid tables
-        const int m = tid + u * T;
-        return NAT ? base + ((long long)m << log2S) : lbase + m;
-    };
-    auto axis_at = [&](int u) { return NAT ? grid_at(u) : (long long)(tid + u * T); };  // pass-axis tables
+    auto grid_at = [&](int u) { return lbase + tid + u * T; };                            // full-grid tables
+    auto axis_at = [&](int u) { return ROWS ? grid_at(u) : (long long)(tid + u * T); };  // pass-axis tables
     if (tr) {
 #pragma unroll
         for (int u = 0; u < E; ++u) v[u] = cscale(v[u], __ldg(tr + grid_at(u)));
@@ -574,7 +574,7 @@ __device__ __forceinline__ void pass_group(const PassArgs<R>& a, long long g, un
             for (int i = t; i < L; i += NT) spec_s[L + i] = __ldg(a.spec2 + i);
     }
 
-    if constexpr (MODE == PM_DOUBLE || MODE == PM_SANDWICH) {
+    if constexpr (MODE == PM_DOUBLE || MODE == PM_SANDWICH || MODE == PM_ROUNDTRIP) {
         // the read-only tables: start their journey to L2 now, before the wait for the previous
         // pass (which writes only the state), so that it overlaps that pass's tail
         if (active) {
@@ -687,7 +687,12 @@ __device__ __forceinline__ void pass_group(const PassArgs<R>& a, long long g, un
         for (int u = 0; u < E; ++u) v[u] = cscale(v[u], a.scale);
         if (active)
             apply_factors<R, E, T, true>(v, tid, base, lbase, a.mid_real, a.mid_cplx, a.mid_ax_cplx, a.mid_ax_real,
-                                         a.axis, a.dim, a.shift, a.nmask, nullptr, key0 ^ 0x2545f491u, log2S);
+                                         a.axis, a.dim, a.shift, a.nmask, nullptr, key0 ^ 0x2545f491u);
+        if (HAS_RED && a.red.n) {
+            if (active)
+                accumulate_line<R, E, T>(a.red, acc, v, a.partner, base, log2S, lbase, tid, a.axis, a.shift, a.nmask);
+            finish_red<NT>(a.red, acc, unsigned(g), ngroups);
+        }
         fft_line_stages<L, E, -1, 0, TWS>(v, tid, line, tw, lsync);
         store_out = true;
     } else if constexpr (MODE == PM_SPECRED) {
@@ -845,7 +850,7 @@ __device__ __forceinline__ void pass_group(const PassArgs<R>& a, long long g, un
         }
     }
     if constexpr (HAS_RED)
-        if (MODE == PM_SPECRED || (a.red.n && (MODE == PM_DOUBLE ? RED_END : !a.red_at_mid)))
+        if (MODE == PM_SPECRED || (a.red.n && MODE != PM_ROUNDTRIP && (MODE == PM_DOUBLE ? RED_END : !a.red_at_mid)))
             finish_red<NT>(a.red, acc, unsigned(g), ngroups);
 }
 
