@@ -141,6 +141,10 @@ struct RecordedPass {
     std::vector<unsigned char> args;
 };
 
+// In the place of a pass axis: the strided virtual axis of a long 1-D axis, whose line-major order its
+// r-space tables take inside a chain (run_chain).
+constexpr int LONG_ROWS = MAX_DIM;
+
 struct qnd_ctx {
     int device = 0;
     cudaStream_t stream = nullptr;
@@ -170,7 +174,7 @@ struct qnd_ctx {
     DevBuf tw_chain;      // 1-D grids the chain kernel takes: its stage twiddles (run_chain1d)
     DevBuf r_dev, p_dev;  // concatenated axes (double)
     DevBuf gradv_dev[MAX_DIM];                // natural layout
-    DevBuf gradv_lm[MAX_DIM][MAX_DIM];        // [component][pass axis] line-major copies
+    DevBuf gradv_lm[MAX_DIM][MAX_DIM + 1];    // [component][pass axis or LONG_ROWS] line-major copies
     DevBuf mask_dev[MAX_DIM];
     DevBuf vpot_dev;      // double, for the energy operator
     std::map<std::tuple<int, int, double, double>, std::unique_ptr<DevBuf>> spec_cache;
@@ -195,7 +199,7 @@ struct qnd_ctx {
     DevBuf finite_slot;                         // QND_CHECK_FINITE: the non-finite count
     std::map<std::tuple<const void*, int, int>, CUtensorMap> tmaps;  // strided-pass TMA views of states
 
-    // A 1-D axis longer than one pass handles: N = n1 n2 (n1 >= 16, n2 <= 4096) as a virtual
+    // A 1-D axis longer than one pass handles: N = n1 n2 (64 to 4096 each) as a virtual
     // n1 x n2 grid transformed in four steps (long_fft). tw_long[v]: the stage twiddles of the
     // length-n1 (v = 0) and length-n2 (v = 1) passes; twf_long / twc_long: the four-step twiddle
     // W_N^{k1 m} and its conjugate at slot k1 n2 + m; p_slot: the momentum of each k-space slot
@@ -204,6 +208,7 @@ struct qnd_ctx {
     int64_t n1 = 0, n2 = 0;
     int lg1 = 0, lg2 = 0;
     DevBuf tw_long[2], twf_long, twc_long, p_slot_dev, long_tmp;
+    DevBuf r_rows, mask_rows;  // the axis and its step mask in LONG_ROWS order
     // Axes longer than 4096 points on grids of several dimensions (emulate_long_pass): per axis the
     // virtual lengths n1 n2, their pass twiddles, the four-step twiddles and their conjugates (at
     // slot k1 n2 + m, as for the 1-D long axis); two scratch states for permutations and copies.
@@ -429,11 +434,12 @@ static inline double clamped_exp(double arg) { return std::exp(arg > MAX_EXP_ARG
 //   RT_VEL    (a[, b]):  exp(min(700,-a Vcap)) exp(-i a V) [* same with b]       complex (integrators.c:209-229)
 //   RT_LENGTH_ADJ (h), RT_VEL_ADJ (a[, b]): the complex conjugates (the adjoints of those factors)
 // Reorder a full-grid array (comps values per point) to line-major order for axis ax: entry
-// lam*L + m holds point m of line lam (the order in which a pass along ax visits the grid).
+// lam*L + m holds point m of line lam (the order in which a pass along ax visits the grid). ax may be
+// LONG_ROWS.
 static std::vector<double> line_major(const qnd_ctx* c, const std::vector<double>& nat, int comps, int ax) {
     if (ax == c->dim - 1) return nat;
-    const int64_t L = c->nr[ax];
-    const int log2S = c->shift[ax];
+    const int64_t L = ax == LONG_ROWS ? c->n1 : c->nr[ax];
+    const int log2S = ax == LONG_ROWS ? c->lg2 : c->shift[ax];
     const int64_t S = int64_t(1) << log2S, nlines = c->n / L;
     std::vector<double> out(nat.size());
     for (int64_t lam = 0; lam < nlines; ++lam) {
@@ -956,6 +962,7 @@ static void launch_pass(qnd_ctx* c, const PassSpec& ps) {
     // registers for the transform
     int kmode = ps.mode;
     if (ps.red.n && ps.mode == PM_SANDWICH) kmode = PM_SANDWICH_RED;
+    if (ps.red.n && ps.mode == PM_ROUNDTRIP) kmode = PM_ROUNDTRIP_RED;
     if (ps.red.n && ps.mode == PM_DOUBLE) kmode = ps.red_at_mid ? PM_DOUBLE_RED : PM_DOUBLE_RED_END;
     // the shape variant: the default while recording (the sweep kernel holds the default shapes)
     const int var = c->recorder ? 0 : (ps.force_shape >= 0 ? ps.force_shape : shape_choice(c, ps, L, log2S, kmode));
@@ -1300,7 +1307,7 @@ static void emulate_long_pass(qnd_ctx* c, const PassSpec& ps) {
 
 // ---------------------------------------------------------------- long axes --
 //
-// A 1-D axis of N = n1 n2 points (n2 = min(4096, N / 16), n1 = N / n2) is transformed in four
+// A 1-D axis of N = n1 n2 points is transformed in four
 // steps over the virtual n1 x n2 grid in which point n1_ n2 + n2_ sits (natural order):
 //   F[k1 + n1 k2] = sum_{n2_} W_{n2}^{n2_ k2} W_N^{n2_ k1} sum_{n1_} W_{n1}^{n1_ k1} psi[n1_ n2 + n2_]
 // i.e. length-n1 transforms along the strided virtual axis, the twiddles W_N^{k1 n2_}, then
@@ -1385,11 +1392,11 @@ static void long_point(qnd_ctx* c, void* psi, const void* treal, const void* tcp
     if (c->fp64)
         launch_point_factors<double>(c->n, static_cast<double2*>(psi), static_cast<const double*>(treal),
                                      static_cast<const double2*>(tcplx), static_cast<const double2*>(pcplx),
-                                     static_cast<const double*>(preal), scale_dev, c->stream);
+                                     long_args(c), static_cast<const double*>(preal), scale_dev, c->stream);
     else
         launch_point_factors<float>(c->n, static_cast<float2*>(psi), static_cast<const float*>(treal),
                                     static_cast<const float2*>(tcplx), static_cast<const float2*>(pcplx),
-                                    static_cast<const float*>(preal), scale_dev, c->stream);
+                                    long_args(c), static_cast<const float*>(preal), scale_dev, c->stream);
     c->kernels_launched++;
     QND_CK(cudaGetLastError());
 }
@@ -1472,7 +1479,10 @@ static std::vector<RedDesc> rspace_red(qnd_ctx* c, const std::vector<ObsItem>& i
     for (auto& it : items) {
         if (it.kind == OB_NORM) add(it.offset, RK_ABS2, WK_ONE, 0, nullptr, c->dNr);
         else if (it.kind == OB_DIPOLE_R)
-            for (int j = 0; j < c->dim; ++j) add(it.offset + j, RK_ABS2, WK_AXIS, j, c->r_dev.as<double>() + c->axoff[j], c->dNr);
+            for (int j = 0; j < c->dim; ++j) {
+                if (lm_axis == LONG_ROWS) add(it.offset + j, RK_ABS2, WK_GRID, 0, c->r_rows.as<double>(), c->dNr);
+                else add(it.offset + j, RK_ABS2, WK_AXIS, j, c->r_dev.as<double>() + c->axoff[j], c->dNr);
+            }
         else if (it.kind == OB_ACCEL)
             for (int j = 0; j < c->dim; ++j) add(it.offset + j, RK_ABS2, WK_GRID, 0, gradv_layout(c, j, lm_axis), -c->dNr);
     }
@@ -1647,8 +1657,10 @@ static void build_field_tables(qnd_ctx* c, const double* field_dev, int64_t nste
     FieldTableArgs fa{};
     fa.conj_from = conj_from;
     fa.field = field_dev;
-    // velocity tables of a long axis: slot order (k-space tables), the 1/n2 of its sandwich pass
-    fa.axes = velocity ? (c->long1d ? c->p_slot_dev.as<double>() : c->p_dev.as<double>()) : c->r_dev.as<double>();
+    // a long axis: velocity tables in slot order (k-space tables), with the 1/n2 of its sandwich pass;
+    // laser phases in the line-major order of its strided virtual axis
+    fa.axes = velocity ? (c->long1d ? c->p_slot_dev.as<double>() : c->p_dev.as<double>())
+                       : (c->long1d ? c->r_rows.as<double>() : c->r_dev.as<double>());
     fa.nsteps = int(nsteps);
     fa.s = c->s;
     fa.dim = c->dim;
@@ -1861,9 +1873,9 @@ static void run_chain(qnd_ctx* c, void* psi, const std::vector<ChainK>& K, const
     }
     if (c->long1d) {
         // four-step sandwiches: length-n1 forward, the length-n2 sandwich pass (twiddles, slot-order
-        // k-space table, conjugate twiddles), then either one length-n1 roundtrip pass (inverse,
-        // the r-space factors in natural order, forward of the next sandwich; FP32) or the
-        // length-n1 inverse and element-wise work in natural order (FP64, reductions, chain end)
+        // k-space table, conjugate twiddles), then one length-n1 roundtrip pass (inverse, the r-space
+        // factors and reductions, forward of the next sandwich) with every table in its line-major
+        // order. The chain's ends work in natural order: element-wise kernels and grid reductions.
         auto point = [&](const Factor& f, int64_t lst, bool mask, const double* scale_dev) {
             const void *tr = nullptr, *tc = nullptr;
             const void* axc[MAX_DIM] = {};
@@ -1879,23 +1891,17 @@ static void run_chain(qnd_ctx* c, void* psi, const std::vector<ChainK>& K, const
             ps.spec_full = 1;
             ps.epi_cplx = c->twc_long.p;
             launch_pass(c, ps);
-            const bool last = i + 1 == NK;
-            const ChainMid& m = last ? post : M[i];
-            // the roundtrip gathers its natural-order tables across the strided virtual axis:
-            // measured 13% faster per step in FP32 at 262144 points, 4% slower in FP64 (where the
-            // separate coalesced element-wise kernel wins)
-            if (!last && !m.red && !c->fp64) {
-                PassSpec r = long_pass(c, 0, PM_ROUNDTRIP, psi, 1.0 / double(c->n1));
-                set_factor(c, m.f, 0, m.lst, &r.mid_real, &r.mid_cplx, r.mid_ax_cplx);
-                if (m.mask) r.mid_ax_real[0] = c->mask_dev[0].p;
-                launch_pass(c, r);
-                continue;
-            }
-            launch_pass(c, long_pass(c, 0, PM_FFT_INV, psi, 1.0 / double(c->n1)));
-            point(m.f, m.lst, m.mask, nullptr);
-            if (m.red) grid_reduce(c, psi, *m.red);
-            if (!last) launch_pass(c, long_pass(c, 0, PM_FFT_FWD, psi, 1.0));
+            if (i + 1 == NK) break;
+            const ChainMid& m = M[i];
+            PassSpec r = long_pass(c, 0, PM_ROUNDTRIP, psi, 1.0 / double(c->n1));
+            set_factor(c, m.f, LONG_ROWS, m.lst, &r.mid_real, &r.mid_cplx, r.mid_ax_cplx);
+            if (m.mask) r.mid_ax_real[0] = c->mask_rows.p;
+            if (m.red) r.red = *m.red;
+            launch_pass(c, r);
         }
+        launch_pass(c, long_pass(c, 0, PM_FFT_INV, psi, 1.0 / double(c->n1)));
+        point(post.f, post.lst, post.mask, nullptr);
+        if (post.red) grid_reduce(c, psi, *post.red);
         return;
     }
     auto finish = [&](PassSpec& ps) {
@@ -2061,9 +2067,9 @@ static void length_steps(qnd_ctx* c, void* psi, int64_t lst0, int64_t n, const R
     std::vector<ChainMid> M;
     std::vector<std::vector<RedDesc>> reds;
     reds.reserve(size_t(n) + 1);
-    auto reductions = [&](int64_t k) -> const RedDesc* {
+    auto reductions = [&](int64_t k, bool inside) -> const RedDesc* {
         if (!red_fn) return nullptr;
-        reds.push_back(red_fn(k, sandwich_last_axis(c, int64_t(K.size()) - 1)));
+        reds.push_back(red_fn(k, c->long1d && inside ? LONG_ROWS : sandwich_last_axis(c, int64_t(K.size()) - 1)));
         if (reds.back().size() > 1) QND_FAIL(QND_EINVAL, "internal: more than one reduction descriptor in a chain");
         return reds.back().empty() ? nullptr : &reds.back()[0];
     };
@@ -2077,7 +2083,7 @@ static void length_steps(qnd_ctx* c, void* psi, int64_t lst0, int64_t n, const R
                 ChainMid b;
                 b.lst = lst - 1;
                 b.mask = masked;
-                b.red = reductions(k - 1);
+                b.red = reductions(k - 1, true);
                 if (b.empty()) {
                     K.back().coef += kk.coef;
                     continue;
@@ -2097,7 +2103,7 @@ static void length_steps(qnd_ctx* c, void* psi, int64_t lst0, int64_t n, const R
     ChainMid post;
     post.lst = lst0 + n - 1;
     post.mask = masked;
-    post.red = reductions(n - 1);
+    post.red = reductions(n - 1, false);
     run_chain(c, psi, K, M, Factor{}, lst0, nullptr, post);
 }
 
@@ -2404,10 +2410,10 @@ static void apply_step_masks(qnd_ctx* c, void* psi) {
 static void apply_table(qnd_ctx* c, void* psi, const void* table) {
     if (c->fp64)
         launch_point_factors<double>(c->n, static_cast<double2*>(psi), nullptr, static_cast<const double2*>(table),
-                                     nullptr, nullptr, nullptr, c->stream);
+                                     nullptr, LongArgs{}, nullptr, nullptr, c->stream);
     else
         launch_point_factors<float>(c->n, static_cast<float2*>(psi), nullptr, static_cast<const float2*>(table),
-                                    nullptr, nullptr, nullptr, c->stream);
+                                    nullptr, LongArgs{}, nullptr, nullptr, c->stream);
     c->kernels_launched++;
     QND_CK(cudaGetLastError());
 }
@@ -2482,11 +2488,11 @@ static void adjoint_run(qnd_ctx* c, const void* psi0, const double* F, int64_t n
     grid_reduce(c, work.p, rj);
     copy_state(c, lam.p, work.p);
     if (c->fp64)
-        launch_point_factors<double>(c->n, lam.as<double2>(), wscaled.as<double>(), nullptr, nullptr, nullptr, nullptr,
-                                     c->stream);
+        launch_point_factors<double>(c->n, lam.as<double2>(), wscaled.as<double>(), nullptr, nullptr, LongArgs{},
+                                     nullptr, nullptr, c->stream);
     else
-        launch_point_factors<float>(c->n, lam.as<float2>(), wscaled.as<float>(), nullptr, nullptr, nullptr, nullptr,
-                                    c->stream);
+        launch_point_factors<float>(c->n, lam.as<float2>(), wscaled.as<float>(), nullptr, nullptr, LongArgs{}, nullptr,
+                                    nullptr, c->stream);
     c->kernels_launched++;
 
     auto kin = [&](double coef) {
@@ -2726,7 +2732,13 @@ static void build_long_axis_nd(qnd_ctx* c, int ax) {
 static void build_long_axis(qnd_ctx* c) {
     const int64_t N = c->nr[0];
     c->long1d = true;
-    c->lg1 = std::max(4, c->lognr[0] - 12);  // n1 >= 16: the strided passes keep 16 values per thread
+    // Two lengths of about the same size (the shorter one strided), 64 to 4096 points each: both virtual
+    // axes then have many lines to spread over the SMs (64 x 4096 gave the contiguous pass of 262144
+    // points 64 CTAs for 148 SMs, 29.6 us). From 2^16 to 2^18 points the contiguous axis takes 256 points,
+    // two radix-16 stages. us per FP64 BM4 step with observables: 2^17 as 512 x 256 101, as 256 x 512 108;
+    // 2^18 as 1024 x 256 117, as 512 x 512 122, as 256 x 1024 125; 2^19 as 512 x 1024 172, as 2048 x 256
+    // 181; 2^20 as 1024 x 1024 276, as 4096 x 256 477.
+    c->lg1 = c->lognr[0] >= 16 && c->lognr[0] <= 18 ? c->lognr[0] - 8 : c->lognr[0] / 2;
     c->lg2 = c->lognr[0] - c->lg1;
     c->n1 = int64_t(1) << c->lg1;
     c->n2 = int64_t(1) << c->lg2;
@@ -2736,6 +2748,7 @@ static void build_long_axis(qnd_ctx* c) {
     c->p_slot.resize(size_t(N));
     for (int64_t i = 0; i < N; ++i) c->p_slot[i] = c->p[0][(i >> c->lg2) + ((i & (c->n2 - 1)) << c->lg1)];
     upload_f64(c, c->p_slot_dev, c->p_slot);
+    upload_f64(c, c->r_rows, line_major(c, c->r[0], 1, LONG_ROWS));
 }
 
 static void build_context(qnd_ctx* c, int dim, const int64_t* nr, const double* dr, const char* integrator,
@@ -3031,11 +3044,11 @@ int qnd_set_gradv(qnd_ctx* ctx, int axis, const double* gradv_host) {
     if (!gradv_host) {
         ctx->gradv[axis].clear();
         ctx->gradv_dev[axis].reset();
-        for (int k = 0; k < MAX_DIM; ++k) ctx->gradv_lm[axis][k].reset();
+        for (int k = 0; k <= MAX_DIM; ++k) ctx->gradv_lm[axis][k].reset();
     } else {
         ctx->gradv[axis].assign(gradv_host, gradv_host + ctx->n);
         upload_f64(ctx, ctx->gradv_dev[axis], ctx->gradv[axis]);
-        for (int k = 0; k < MAX_DIM; ++k) ctx->gradv_lm[axis][k].reset();
+        for (int k = 0; k <= MAX_DIM; ++k) ctx->gradv_lm[axis][k].reset();
     }
     QND_API_END
 }
@@ -3049,9 +3062,11 @@ int qnd_set_mask_axis(qnd_ctx* ctx, int axis, const double* mask_host) {
     if (!mask_host) {
         ctx->mask[axis].clear();
         ctx->mask_dev[axis].reset();
+        ctx->mask_rows.reset();
     } else {
         ctx->mask[axis].assign(mask_host, mask_host + ctx->nr[axis]);
         upload_real(ctx, ctx->mask_dev[axis], ctx->mask[axis]);
+        if (ctx->long1d) upload_real(ctx, ctx->mask_rows, line_major(ctx, ctx->mask[axis], 1, LONG_ROWS));
     }
     QND_API_END
 }

@@ -157,11 +157,12 @@ template <typename R> void launch_long_twiddle(const LongArgs& a, cplx_t<R>* psi
 // to_natural: out[k1 + N1 k2] = in[k1 N2 + k2]; otherwise the inverse permutation
 template <typename R> void launch_long_transpose(const LongArgs& a, const cplx_t<R>* in, cplx_t<R>* out, int to_natural,
                                                  cudaStream_t st);
-// Point-wise factors of a 1-D state in natural order: real table, complex table, per-axis complex
-// table, real per-axis table (the mask), device scalar; any may be null.
+// Point-wise factors of a state in natural order: real table, complex table, the laser phases pc of a
+// long 1-D axis (in the line-major order of its strided virtual axis, lengths in pc_order), real
+// per-axis table (the mask), device scalar; any may be null.
 template <typename R> void launch_point_factors(long long n, cplx_t<R>* psi, const R* tr, const cplx_t<R>* tc,
-                                                const cplx_t<R>* pc, const R* pr, const double* scale_dev,
-                                                cudaStream_t st);
+                                                const cplx_t<R>* pc, const LongArgs& pc_order, const R* pr,
+                                                const double* scale_dev, cudaStream_t st);
 // psi *= prod_j mask_j[index along axis j] over the axes whose mask is set (natural layout)
 template <typename R> void launch_apply_masks(long long n, cplx_t<R>* psi, int dim, const int* shift,
                                               const long long* nmask, const R* const* masks, cudaStream_t st);

@@ -38,13 +38,13 @@ def test_real_time_chains(qnd_lib, n, integ, steps):
     want = o.run_length(a, F, names)
     got = g.run_length(st, F, names)
     assert rel(st.download(), a) < 1e-12 * max(1, steps / 10)
-    np.testing.assert_allclose(got, want, rtol=1e-11, atol=1e-13)
+    assert np.all(np.abs(got - want) <= 1e-11 * np.max(np.abs(want), axis=0))  # the dipole crosses zero
     alpha = np.random.default_rng(1).standard_normal((steps, 1)) * 0.05
     a, st = psi0.copy(), g.state(psi0)
     want = o.run_velocity(a, F, alpha, names)
     got = g.run_velocity(st, F, alpha, names)
     assert rel(st.download(), a) < 1e-12 * max(1, steps / 10)
-    np.testing.assert_allclose(got, want, rtol=1e-11, atol=1e-13)
+    assert np.all(np.abs(got - want) <= 1e-11 * np.max(np.abs(want), axis=0))  # the dipole crosses zero
 
 
 @pytest.mark.parametrize("n", [64, 128, 512, 4096])
