@@ -51,28 +51,27 @@ __global__ void __launch_bounds__(L / E, 1) qnd_chain1d_kernel(const __grid_cons
     static_assert(T >= 32 && T % 32 == 0, "whole warps");
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ double red_s[T / 32][MAX_RED];
+    __shared__ RedShared<T> red_sh;
     __shared__ double sum_s[MAX_RED];
     __shared__ double coef_s[2 * GS_MAXK];
     V* tw = reinterpret_cast<V*>(smem_raw);
     V* line = tw + SH::TW;
     const int tid = threadIdx.x;
     const LineSync<T> lsync{1};
-    const int shift1 = 0;
-    const long long nmask1 = L - 1;
 
     for (int i = tid; i < (sizeof(R) == 8 ? SH::P::twb_size() : SH::P::tw_size()); i += T) tw[i] = a.tw[i];
     V v[E];
 #pragma unroll
     for (int u = 0; u < E; ++u) v[u] = a.psi[tid + u * T];
-    __syncthreads();  // twiddles visible
+    load_red_rows<T>(a.red, 0, red_sh);
+    __syncthreads();  // twiddles and reductions visible
 
     // the point-wise factor `mid` (a full-grid table) with the laser phases at `laser`, the step mask
     // and a device scalar
     auto factors = [&](int mid, int laser, bool mask, const double* scale, uint32_t key) {
-        const V* axc[1] = {laser >= 0 ? a.field + laser : nullptr};
-        const R* axr[1] = {mask ? a.mask : nullptr};
-        apply_factors<R, E, T>(v, tid, 0, 0, mid >= 0 ? a.mid_real[mid] : nullptr, mid >= 0 ? a.mid_cplx[mid] : nullptr,
-                               axc, axr, 0, 1, &shift1, &nmask1, scale, key);
+        apply_tables<R, E, T>(v, tid, 0, mid >= 0 ? a.mid_real[mid] : nullptr, mid >= 0 ? a.mid_cplx[mid] : nullptr,
+                              laser >= 0 ? a.field + laser : nullptr, mask ? a.mask : nullptr, false, V{},
+                              scale != nullptr, scale ? R(*scale) : R(1), key);
     };
     factors(a.pre_mid, a.pre_laser, false, a.pre_scale, mix32(a.seed) ^ 0x51ed270bu);
 
@@ -91,12 +90,18 @@ __global__ void __launch_bounds__(L / E, 1) qnd_chain1d_kernel(const __grid_cons
         fft_line_stages<L, E, +1, 0, true>(v, tid, line, tw, lsync);
         factors(op.mid, op.laser, op.mask != 0, nullptr, key ^ 0x2545f491u);
         if (op.obs >= 0) {
-            double acc[MAX_RED];
-#pragma unroll
-            for (int k = 0; k < MAX_RED; ++k) acc[k] = 0.0;
-            accumulate_line<R, E, T>(a.red, acc, v, static_cast<const V*>(nullptr), 0, 0, 0, tid, 0, &shift1, &nmask1);
-            cta_sums<T>(acc, a.red.n, red_s, sum_s);
-            if (tid < a.red.n) a.red.out[op.obs + tid] = sum_s[tid] * a.red.scale[tid];
+#pragma unroll 1
+            for (int k = 0; k < a.red.n; ++k) {
+                const double s = warp_sum(line_sum<R, E, T>(red_sh.row[k], v, static_cast<const V*>(nullptr), 0, 0, 0, tid));
+                if ((tid & 31) == 0) red_sh.s[tid >> 5][k] = s;
+            }
+            __syncthreads();
+            if (tid < a.red.n) {
+                double s = 0.0;
+                for (int w = 0; w < T / 32; ++w) s += red_sh.s[w][tid];
+                a.red.out[op.obs + tid] = s * a.red.scale[tid];
+            }
+            __syncthreads();  // the warps' sums are read
         }
         if (op.gs) {
             // v = psi - sum_k <psi_k|psi> psi_k, then v / ||v|| (QuantumND_imag.c:280-310)

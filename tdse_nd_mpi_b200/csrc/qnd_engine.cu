@@ -628,6 +628,15 @@ template <typename R> static void fill_args(qnd_ctx* c, const PassSpec& ps, Pass
         a.ax_real[k] = static_cast<const R*>(ps.ax_real[k]);
     }
     a.ax_in_prologue = ps.ax_in_prologue;
+    a.sandwiches = ps.mode == PM_DOUBLE ? 2 : 1;
+    bool ax = false, axr = false, mid = a.mid_real || a.mid_cplx;
+    for (int k = 0; k < MAX_DIM; ++k) {
+        ax = ax || a.ax_cplx[k];
+        axr = axr || a.ax_real[k];
+        mid = mid || a.mid_ax_cplx[k] || a.mid_ax_real[k];
+    }
+    a.points = (a.pro_real || a.pro_cplx || a.pro_scale_dev || (ax && a.ax_in_prologue) ? 1 : 0) | (mid ? 2 : 0) |
+               (a.epi_real || a.epi_cplx || (ax && !a.ax_in_prologue) || axr ? 4 : 0);
     a.scale = R(ps.scale);
     a.apply_acc = ps.apply_acc;
     a.apply_vtab = ps.apply_vtab;
@@ -846,8 +855,8 @@ static void load_shape_table() {
     std::fclose(f);
 }
 
-static int shape_choice(qnd_ctx* c, const PassSpec& ps, int L, int log2S, int kmode) {
-    const int mode = pass_base_mode(kmode);
+static int shape_choice(qnd_ctx* c, const PassSpec& ps, int L, int log2S) {
+    const int mode = ps.mode, kmode = pass_kernel_mode(mode, ps.red.n > 0);
     if (ps.vL || (mode != PM_SANDWICH && mode != PM_DOUBLE) || L < 256 || L > 2048) return 0;
     const bool strided = log2S > 0;
     if (const char* f = std::getenv("QND_SHAPE")) {
@@ -865,7 +874,7 @@ static int shape_choice(qnd_ctx* c, const PassSpec& ps, int L, int log2S, int km
         if (tt != g_shape_table.end()) {
             cudaDeviceProp prop{};
             if (cudaGetDeviceProperties(&prop, c->device) == cudaSuccess && g_shape_table_device == prop.name &&
-                tt->second >= 0 && tt->second < NSHAPES && lookup_pass(c->fp64, L, strided, mode, tt->second).fn) {
+                tt->second >= 0 && tt->second < NSHAPES && lookup_pass(c->fp64, L, strided, kmode, tt->second).fn) {
                 g_shape[key] = tt->second;
                 return tt->second;
             }
@@ -892,7 +901,7 @@ static int shape_choice(qnd_ctx* c, const PassSpec& ps, int L, int log2S, int km
     int choice = 0;
     for (int v = 0; v < NSHAPES; ++v) {
         ms[v] = -1.f;
-        if (!lookup_pass(c->fp64, L, strided, mode, v).fn) continue;
+        if (!lookup_pass(c->fp64, L, strided, kmode, v).fn) continue;
         t.force_shape = v;
         launch_pass(c, t);
         QND_CK(cudaEventRecord(e0, c->stream));
@@ -960,12 +969,9 @@ static void launch_pass(qnd_ctx* c, const PassSpec& ps) {
     const bool strided = log2S > 0;
     // passes that reduce run the instantiation that carries the reduction code; the others keep its
     // registers for the transform
-    int kmode = ps.mode;
-    if (ps.red.n && ps.mode == PM_SANDWICH) kmode = PM_SANDWICH_RED;
-    if (ps.red.n && ps.mode == PM_ROUNDTRIP) kmode = PM_ROUNDTRIP_RED;
-    if (ps.red.n && ps.mode == PM_DOUBLE) kmode = ps.red_at_mid ? PM_DOUBLE_RED : PM_DOUBLE_RED_END;
+    const int kmode = pass_kernel_mode(ps.mode, ps.red.n > 0);
     // the shape variant: the default while recording (the sweep kernel holds the default shapes)
-    const int var = c->recorder ? 0 : (ps.force_shape >= 0 ? ps.force_shape : shape_choice(c, ps, L, log2S, kmode));
+    const int var = c->recorder ? 0 : (ps.force_shape >= 0 ? ps.force_shape : shape_choice(c, ps, L, log2S));
     const PassKernelInfo info = lookup_pass(c->fp64, L, strided, kmode, var);
     if (!info.fn) QND_FAIL(QND_EINVAL, "internal: no pass kernel for L=%d, mode %d, shape %d", L, kmode, var);
     if (var != 0 && info.E != lookup_pass(c->fp64, L, strided, kmode, 0).E)
@@ -975,8 +981,7 @@ static void launch_pass(qnd_ctx* c, const PassSpec& ps) {
     if (c->recorder) {
         // qnd_run_length_sweep: the arguments this launch would get (per-thread staging: the sweep
         // kernel takes its arguments from device memory), kept for the persistent kernel
-        if (!sweep_length_ok(L) || ps.vL || (kmode != PM_SANDWICH && kmode != PM_SANDWICH_RED && kmode != PM_DOUBLE &&
-                                             kmode != PM_DOUBLE_RED && kmode != PM_DOUBLE_RED_END))
+        if (!sweep_length_ok(L) || ps.vL || (kmode != PM_SANDWICH && kmode != PM_SANDWICH_RED))
             QND_FAIL(QND_EUNSUPPORTED, "qnd_run_length_sweep: a pass of line length %d, mode %d is outside the "
                                        "sweep kernel (axis lengths 128 to 1024)", L, kmode);
         RecordedPass rp;
@@ -1841,6 +1846,10 @@ static void run_chain1d(qnd_ctx* c, void* psi, const std::vector<ChainK>& K, con
             op.mask = m.mask && a.mask;
             if (m.red) {
                 if (!a.red.n) {
+                    // the kernel needs no scratch, but a chunk's graph key holds the scratch addresses:
+                    // allocated in the first chunk as by a pass, so that a member captures the same
+                    // chunk alone and in a batch (a graph keeps the FP32 dither streams of its capture)
+                    ensure_red_scratch(c, 1);
                     a.red = *m.red;
                     set_red_axes(c, a.red);
                 }

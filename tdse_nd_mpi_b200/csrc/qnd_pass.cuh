@@ -36,6 +36,8 @@
 
 #include "qnd_fft.cuh"
 
+#include <type_traits>
+
 namespace qnd {
 
 constexpr int MAX_RED = 8;
@@ -47,23 +49,23 @@ enum : int {
     PM_FFT_INV = 2,
     PM_SPECRED = 3,
     PM_APPLY = 4,
-    PM_DOUBLE = 5,
+    PM_DOUBLE = 5,        // runs the kernels of PM_SANDWICH with four turns
     PM_ROUNDTRIP = 6,
-    PM_SANDWICH_RED = 7,  // PM_SANDWICH / PM_DOUBLE with fused reductions: separate instantiations, so that
-    PM_DOUBLE_RED = 8,    // the passes without reductions (most of a chain) keep their registers for the FFT;
-    PM_DOUBLE_RED_END = 9,  // PM_DOUBLE_RED reduces between its sandwiches (a step boundary), _END after both
-    PM_ROUNDTRIP_RED = 10,
-    PM_NMODES = 11
+    PM_SANDWICH_RED = 7,  // with fused reductions: separate instantiations, so that the passes without them
+    PM_ROUNDTRIP_RED = 8, // (most of a chain) keep their registers for the transform
+    PM_NMODES = 9
 };
-// The transform structure of a mode (the reducing variants share their base mode's) and whether the
-// mode can carry reductions at all.
+// The transform structure of a kernel's mode (the reducing variants share their base mode's), whether the
+// mode can carry reductions at all, and the kernel mode of a pass.
 __host__ __device__ constexpr int pass_base_mode(int m) {
-    return m == PM_SANDWICH_RED ? PM_SANDWICH
-           : (m == PM_DOUBLE_RED || m == PM_DOUBLE_RED_END) ? PM_DOUBLE
-           : m == PM_ROUNDTRIP_RED ? PM_ROUNDTRIP : m;
+    return m == PM_SANDWICH_RED ? PM_SANDWICH : (m == PM_ROUNDTRIP_RED ? PM_ROUNDTRIP : m);
 }
 __host__ __device__ constexpr bool pass_mode_reduces(int m) {
-    return m == PM_SANDWICH_RED || m == PM_ROUNDTRIP_RED || m == PM_DOUBLE_RED || m == PM_DOUBLE_RED_END || m == PM_SPECRED || m == PM_APPLY;
+    return m == PM_SANDWICH_RED || m == PM_ROUNDTRIP_RED || m == PM_SPECRED || m == PM_APPLY;
+}
+__host__ __device__ constexpr int pass_kernel_mode(int m, bool reduces) {
+    return (m == PM_SANDWICH || m == PM_DOUBLE) ? (reduces ? PM_SANDWICH_RED : PM_SANDWICH)
+           : m == PM_ROUNDTRIP ? (reduces ? PM_ROUNDTRIP_RED : PM_ROUNDTRIP) : m;
 }
 // |v|^2 w, Re(conj(partner) v) w, or (element-wise grid reductions only) Im(conj(partner) v) w and
 // the count of elements with a non-finite part
@@ -111,6 +113,8 @@ template <typename R> struct PassArgs {
     const V* mid_ax_cplx[MAX_DIM];
     const R* mid_ax_real[MAX_DIM];  // PM_DOUBLE: per-axis real factors between the sandwiches (step mask)
     int red_at_mid;                 // PM_DOUBLE: reduce the state between the sandwiches, not at the end
+    int sandwiches;                 // of a propagating pass: 1 or 2
+    int points;                     // bits of the places with factors: 1 before, 2 between the sandwiches, 4 after
     const R* epi_real;
     const V* epi_cplx;
     const V* ax_cplx[MAX_DIM];   // per-axis factors (laser phases, step mask) applied ...
@@ -299,68 +303,67 @@ __device__ __forceinline__ void accumulate_red(const RedDesc& rd, double* acc, V
     }
 }
 
-// Reductions over the E values a thread holds of one line (m = tid + u*T), accumulator-outer: for
-// each accumulator the weights are either a per-line scalar (weight 1, or a weight along another
-// axis) or a row read with stride T (a weight along the pass axis, or the line's row of a line-major
-// full-grid table), so one loop serves both; |v|^2 is recomputed per accumulator (two FMAs) rather
-// than held in E extra FP64 registers.
+// A fused reduction's accumulators in shared memory, where they are indexed at run time: the loop over
+// them is rolled. With a copy of the sums for each of the MAX_RED accumulators and each weight kind, a
+// reducing 1024-point pass held 175 KB (FP64) to 232 KB (FP32) of code, and a launch finds the
+// instruction caches cold.
+struct RedRow {
+    const double* w;  // weights: none (null), one for the line at w[(base >> shift) & mask], or a row
+    long long mask;
+    int shift;
+    int how;          // 0 none, 1 one for the line, 2 a row over the pass axis, 3 a row of a line-major table
+    int bilinear;
+};
+template <int NT> struct RedShared {
+    static constexpr int NW = NT / 32 > 0 ? NT / 32 : 1;
+    RedRow row[MAX_RED];
+    double s[NW][MAX_RED];
+    int is_last;
+};
+
+// The descriptor's accumulators for a pass along `axis` into shared memory, by the first threads
+// (compile-time indices into the argument); visible after a CTA barrier.
+template <int NT> __device__ __forceinline__ void load_red_rows(const RedDesc& rd, int axis, RedShared<NT>& sh) {
+#pragma unroll
+    for (int k = 0; k < MAX_RED; ++k)
+        if (int(threadIdx.x) == k && k < rd.n) {
+            const int wk = rd.wkind[k];
+            sh.row[k] = RedRow{rd.wtab[k], rd.wmask[k], rd.wshift[k],
+                               wk == WK_GRID ? 3 : (wk == WK_AXIS ? (rd.waxis[k] == axis ? 2 : 1) : 0),
+                               rd.kind[k] == RK_BILIN};
+        }
+}
+
+// One accumulator's sum over the E values a thread holds of one line (m = tid + u*T).
 template <typename R, int E, int T>
-__device__ __forceinline__ void accumulate_line(const RedDesc& rd, double* acc, const cplx_t<R>* v,
-                                                const cplx_t<R>* partner, long long base, int log2S, long long lbase,
-                                                int tid, int axis, const int* shift, const long long* nmask) {
+__device__ __forceinline__ double line_sum(const RedRow& r, const cplx_t<R>* v, const cplx_t<R>* partner,
+                                           long long base, int log2S, long long lbase, int tid) {
+    const double* __restrict__ row = r.how == 2 ? r.w + tid : (r.how == 3 ? r.w + lbase + tid : nullptr);
+    double sum = 0.0;
+    if (!r.bilinear) {
+        if (row) {
 #pragma unroll
-    for (int k = 0; k < MAX_RED; ++k) {
-        if (k >= rd.n) break;
-        double sum = 0.0;
-        const int wk = rd.wkind[k];
-        const double* __restrict__ wt = rd.wtab[k];
-        if (rd.kind[k] == RK_ABS2) {
-            const double* __restrict__ row = nullptr;  // stride-T weights of this line
-            double wl = 1.0;                           // or one weight for the whole line
-            if (wk == WK_GRID) {
-                row = wt + lbase + tid;
-            } else if (wk == WK_AXIS) {
-                if (rd.waxis[k] == axis) row = wt + tid;
-                else wl = __ldg(wt + ((base >> rd.wshift[k]) & rd.wmask[k]));
-            }
-            if (row) {
-#pragma unroll
-                for (int u = 0; u < E; ++u) {
-                    const double x = v[u].x, y = v[u].y;
-                    sum = fma(fma(x, x, y * y), __ldg(row + u * T), sum);
-                }
-            } else {
-#pragma unroll
-                for (int u = 0; u < E; ++u) {
-                    const double x = v[u].x, y = v[u].y;
-                    sum += fma(x, x, y * y);
-                }
-                sum *= wl;
+            for (int u = 0; u < E; ++u) {
+                const double x = v[u].x, y = v[u].y;
+                sum = fma(fma(x, x, y * y), __ldg(row + u * T), sum);
             }
         } else {
-            // the weights' row and their step along it, or no weights (one branch for the whole line)
-            const double* __restrict__ row = nullptr;
-            int step = T;
-            if (wk == WK_GRID) {
-                row = wt + lbase + tid;
-            } else if (wk == WK_AXIS) {
-                if (rd.waxis[k] == axis) row = wt + tid;
-                else { row = wt + ((base >> rd.wshift[k]) & rd.wmask[k]); step = 0; }
-            }
-            auto bilin = [&](int u) {
-                const cplx_t<R> p = partner[base + ((long long)(tid + u * T) << log2S)];
-                return double(p.x) * double(v[u].x) + double(p.y) * double(v[u].y);
-            };
-            if (row) {
 #pragma unroll
-                for (int u = 0; u < E; ++u) sum += bilin(u) * __ldg(row + u * step);
-            } else {
-#pragma unroll
-                for (int u = 0; u < E; ++u) sum += bilin(u);
+            for (int u = 0; u < E; ++u) {
+                const double x = v[u].x, y = v[u].y;
+                sum += fma(x, x, y * y);
             }
         }
-        acc[k] += sum;
+    } else {
+        const int step = row ? T : 0;
+        const double one = 1.0;
+#pragma unroll
+        for (int u = 0; u < E; ++u) {
+            const cplx_t<R> p = partner[base + ((long long)(tid + u * T) << log2S)];
+            sum += (double(p.x) * double(v[u].x) + double(p.y) * double(v[u].y)) * (row ? __ldg(row + u * step) : one);
+        }
     }
+    return r.how == 1 ? sum * __ldg(r.w + ((base >> r.shift) & r.mask)) : sum;
 }
 
 // Warm L2 with the line-major rows a pass will read later (a full-grid table), one 128-byte
@@ -373,32 +376,24 @@ template <int L, int T, typename X> __device__ __forceinline__ void prefetch_row
     for (int q = tid; q < NLINES; q += T) asm volatile("prefetch.global.L2 [%0];" ::"l"(p + 128 * q));
 }
 
-// Block reduction of acc[0..n) into partials, then the last CTA sums the partials in order.
+// Every warp's sums sh.s[warp][0..n) into partials, then the last CTA sums the partials in order.
 // blk / nblk: this CTA's group and the number of groups (the grid, or a persistent kernel's groups
 // of one pass).
 template <int NT>
-__device__ __forceinline__ void finish_red(const RedDesc& rd, double* acc, unsigned blk, unsigned nblk) {
-    constexpr int NW = NT / 32 > 0 ? NT / 32 : 1;
-    __shared__ double red_s[NW][MAX_RED];
-    __shared__ int is_last;
+__device__ __forceinline__ void finish_red(const RedDesc& rd, RedShared<NT>& sh, unsigned blk, unsigned nblk) {
+    constexpr int NW = RedShared<NT>::NW;
     const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
-#pragma unroll
-    for (int k = 0; k < MAX_RED; ++k) {
-        if (k >= rd.n) break;
-        double s = warp_sum(acc[k]);
-        if (lane == 0) red_s[wid][k] = s;
-    }
     __syncthreads();
     if (t < rd.n) {
         double s = 0.0;
-        for (int w = 0; w < NW; ++w) s += red_s[w][t];
+        for (int w = 0; w < NW; ++w) s += sh.s[w][t];
         rd.partials[(long long)blk * MAX_RED + t] = s;
     }
     __threadfence();
     __syncthreads();
-    if (t == 0) is_last = (atomicAdd(rd.counter, 1u) == nblk - 1);
+    if (t == 0) sh.is_last = (atomicAdd(rd.counter, 1u) == nblk - 1);
     __syncthreads();
-    if (!is_last) return;
+    if (!sh.is_last) return;
     __threadfence();
     // every accumulator in one sweep over the partials (one round of L2 loads, one barrier): the
     // last CTA's tail is the critical path of the pass. Per accumulator the order of the sums is
@@ -416,53 +411,56 @@ __device__ __forceinline__ void finish_red(const RedDesc& rd, double* acc, unsig
     for (int k = 0; k < MAX_RED; ++k) {
         if (k >= rd.n) break;
         const double ws = warp_sum(s[k]);
-        if (lane == 0) red_s[wid][k] = ws;
+        if (lane == 0) sh.s[wid][k] = ws;
     }
     __syncthreads();
     if (t < rd.n) {
         double tot = 0.0;
-        for (int w = 0; w < NW; ++w) tot += red_s[w][t];
+        for (int w = 0; w < NW; ++w) tot += sh.s[w][t];
         tot *= rd.scale[t];
         rd.out[t] = rd.accumulate ? rd.out[t] + tot : tot;
     }
     if (t == 0) *rd.counter = 0u;
 }
+// The same from each thread's accumulators acc[0..n).
 template <int NT> __device__ __forceinline__ void finish_red(const RedDesc& rd, double* acc) {
-    finish_red<NT>(rd, acc, blockIdx.x, gridDim.x);
+    __shared__ RedShared<NT> sh;
+#pragma unroll
+    for (int k = 0; k < MAX_RED; ++k) {
+        if (k >= rd.n) break;
+        const double s = warp_sum(acc[k]);
+        if ((threadIdx.x & 31) == 0) sh.s[threadIdx.x >> 5][k] = s;
+    }
+    finish_red<NT>(rd, sh, blockIdx.x, gridDim.x);
 }
 
-// Point-wise r-space factors on the E values a thread holds of one line: a full-grid table
-// (line-major: entry lbase + m), per-axis complex factors (the pass axis per element, the other
-// axes once per line), per-axis real factors and a scalar.
-// ROWS: the per-axis tables are rows of full tables in line-major order (entry lbase + m) too, not
-// tables over the position m (the strided virtual axis of a long 1-D axis).
-template <typename R, int E, int T, bool ROWS = false>
-__device__ __forceinline__ void apply_factors(cplx_t<R>* v, int tid, long long base, long long lbase,
-                                              const R* __restrict__ tr, const cplx_t<R>* __restrict__ tc,
-                                              const cplx_t<R>* const* axc, const R* const* axr, int axis, int dim,
-                                              const int* shift, const long long* nmask, const double* scale_dev,
-                                              uint32_t key) {
-    using V = cplx_t<R>;
-    V lf = fone<V>();
-    R lr = R(1);
-    bool use_lf = false, use_lr = false;
-    // the pass axis' tables picked by a compile-time index (no run-time indexing of the argument
-    // arrays, which would copy them to local memory)
-    const V* __restrict__ pc = nullptr;
-    const R* __restrict__ pr = nullptr;
-#pragma unroll
-    for (int k = 0; k < MAX_DIM; ++k) {
-        if (k >= dim) break;  // the grid's axes only (a 2-D pass runs two turns of the six)
-        if (k == axis) {
-            if (axc) pc = axc[k];
-            if (axr) pr = axr[k];
-            continue;
-        }
-        const long long ik = (base >> shift[k]) & nmask[k];
-        if (axc && axc[k]) { lf = fcompose(lf, axc[k][ik]); use_lf = true; }
-        if (axr && axr[k]) { lr *= axr[k][ik]; use_lr = true; }
+// The fused reductions of a pass: every line's values, the CTA's sums, the grid's.
+template <typename R, int E, int T, int NT>
+__device__ __forceinline__ void reduce_lines(const RedDesc& rd, RedShared<NT>& sh, const cplx_t<R>* v, bool active,
+                                             const cplx_t<R>* partner, long long base, int log2S, long long lbase,
+                                             int tid, int axis, unsigned blk, unsigned nblk) {
+    load_red_rows<NT>(rd, axis, sh);
+    __syncthreads();
+#pragma unroll 1
+    for (int k = 0; k < rd.n; ++k) {
+        double s = 0.0;
+        if (active) s = line_sum<R, E, T>(sh.row[k], v, partner, base, log2S, lbase, tid);
+        s = warp_sum(s);
+        if ((threadIdx.x & 31) == 0) sh.s[threadIdx.x >> 5][k] = s;
     }
-    if (scale_dev) { lr *= R(*scale_dev); use_lr = true; }
+    finish_red<NT>(rd, sh, blk, nblk);
+}
+
+// Point-wise r-space factors on the E values a thread holds of one line: full-grid tables tr (real) and
+// tc (complex; line-major: entry lbase + m), the factors pc and pr along the pass axis (entry m), and for
+// the whole line lf (the composed complex factors of the other axes) and lr (their real factors and a
+// scalar). ROWS: pc and pr are rows of full tables in line-major order (entry lbase + m) too (the strided
+// virtual axis of a long 1-D axis).
+template <typename R, int E, int T, bool ROWS = false>
+__device__ __forceinline__ void apply_tables(cplx_t<R>* v, int tid, long long lbase, const R* __restrict__ tr,
+                                             const cplx_t<R>* __restrict__ tc, const cplx_t<R>* __restrict__ pc,
+                                             const R* __restrict__ pr, bool use_lf, cplx_t<R> lf, bool use_lr, R lr,
+                                             uint32_t key) {
     // One loop over the thread's elements per factor that is set, so that each loop is free of
     // branches and its table reads go out together: with the tests inside one loop over the elements
     // every read waited for the one before it, and the factor between the sandwiches of a 1024-point
@@ -532,8 +530,8 @@ __device__ __forceinline__ void pass_group(const PassArgs<R>& a, long long g, un
     constexpr bool TMA = SK == 2;
     constexpr int MODE = pass_base_mode(KMODE);
     constexpr bool HAS_RED = pass_mode_reduces(KMODE);
-    // two-sandwich passes: reductions between the sandwiches, or after both (compile-time)
-    constexpr bool RED_MID = KMODE == PM_DOUBLE_RED, RED_END = KMODE == PM_DOUBLE_RED_END;
+    constexpr bool PROPAGATE = MODE == PM_SANDWICH;
+    constexpr bool ONE_TRANSFORM = sizeof(R) == 8 && L >= 1024;  // see the sandwich below
     using V = cplx_t<R>;
     using SH = PassShape<R, L, VAR>;
     constexpr int E = SH::E, T = SH::T, G = SH::G, NT = SH::NT, LS = SH::LS;
@@ -567,14 +565,14 @@ __device__ __forceinline__ void pass_group(const PassArgs<R>& a, long long g, un
     // spectral rows to shared memory (read-only tables: before the wait for the previous pass);
     // visible after the CTA barrier that precedes the first transform
     const bool spec_row = a.spec && !a.spec_full;
-    if constexpr (SH::SPEC_SMEM && (MODE == PM_DOUBLE || MODE == PM_SANDWICH)) {
+    if constexpr (SH::SPEC_SMEM && PROPAGATE) {
         if (spec_row)
             for (int i = t; i < L; i += NT) spec_s[i] = __ldg(a.spec + i);
-        if (MODE == PM_DOUBLE && a.spec2)
+        if (a.spec2)
             for (int i = t; i < L; i += NT) spec_s[L + i] = __ldg(a.spec2 + i);
     }
 
-    if constexpr (MODE == PM_DOUBLE || MODE == PM_SANDWICH || MODE == PM_ROUNDTRIP) {
+    if constexpr (PROPAGATE || MODE == PM_ROUNDTRIP) {
         // the read-only tables: start their journey to L2 now, before the wait for the previous
         // pass (which writes only the state), so that it overlaps that pass's tail
         if (active) {
@@ -583,13 +581,19 @@ __device__ __forceinline__ void pass_group(const PassArgs<R>& a, long long g, un
             if (a.mid_real) prefetch_row_l2<L, T>(a.mid_real + lbase, tid);
             if (a.epi_cplx) prefetch_row_l2<L, T>(a.epi_cplx + lbase, tid);
             if (a.epi_real) prefetch_row_l2<L, T>(a.epi_real + lbase, tid);
-            if constexpr (HAS_RED)
-                for (int k = 0; k < a.red.n; ++k)
-                    if (a.red.wkind[k] == WK_GRID) prefetch_row_l2<L, T>(a.red.wtab[k] + lbase, tid);
+            if constexpr (HAS_RED) {
+#pragma unroll
+                for (int k = 0; k < MAX_RED; ++k)
+                    if (k < a.red.n && a.red.wkind[k] == WK_GRID) prefetch_row_l2<L, T>(a.red.wtab[k] + lbase, tid);
+            }
         }
     }
 
     wait();
+
+    using RS = std::conditional_t<HAS_RED, RedShared<NT>, char>;
+    __shared__ RS red_sh;
+    (void)red_sh;
 
     V v[E];
     if constexpr (STRIDED) {
@@ -624,12 +628,11 @@ __device__ __forceinline__ void pass_group(const PassArgs<R>& a, long long g, un
                 // finishes it and resets the counter.
                 mbar_wait_bounded(&tma_bar, 0, 1 << 20);
                 if (t == 0 && a.err) atomicExch(a.err, 1);
-                if (HAS_RED && (MODE == PM_SPECRED || a.red.n)) {
-                    double none[MAX_RED];
-#pragma unroll
-                    for (int k = 0; k < MAX_RED; ++k) none[k] = 0.0;
-                    finish_red<NT>(a.red, none, unsigned(g), ngroups);
-                }
+                if constexpr (HAS_RED)
+                    if (MODE == PM_SPECRED || a.red.n) {
+                        for (int k = t; k < RedShared<NT>::NW * MAX_RED; k += NT) red_sh.s[k / MAX_RED][k % MAX_RED] = 0.0;
+                        finish_red<NT>(a.red, red_sh, unsigned(g), ngroups);
+                    }
                 return;
             }
 #pragma unroll
@@ -657,150 +660,141 @@ __device__ __forceinline__ void pass_group(const PassArgs<R>& a, long long g, un
         if constexpr (TWS) __syncthreads();  // twiddles visible
     }
 
-    constexpr bool PROPAGATE = MODE == PM_SANDWICH || MODE == PM_DOUBLE;
-    if constexpr (PROPAGATE) {
-        if (active && (a.pro_real || a.pro_cplx || a.pro_scale_dev || a.ax_in_prologue))
-            apply_factors<R, E, T>(v, tid, base, lbase, a.pro_real, a.pro_cplx, a.ax_in_prologue ? a.ax_cplx : nullptr,
-                                   nullptr, a.axis, a.dim, a.shift, a.nmask, a.pro_scale_dev, key0 ^ 0x51ed270bu);
-    }
-    if constexpr (STRIDED) {
-        if constexpr (!TMA) lsync();  // staged inputs read before the exchanges reuse the buffer
-    }
+    if constexpr (STRIDED && !TMA) lsync();  // staged inputs read before the exchanges reuse the buffer
 
-    double acc[MAX_RED];
+    auto reduce = [&] {
+        if constexpr (HAS_RED)
+            reduce_lines<R, E, T, NT>(a.red, red_sh, v, active, a.partner, base, log2S, lbase, tid, a.axis, unsigned(g),
+                                      ngroups);
+    };
+    auto conjugate = [&] {
 #pragma unroll
-    for (int k = 0; k < MAX_RED; ++k) acc[k] = 0.0;
+        for (int u = 0; u < E; ++u) v[u].y = -v[u].y;
+    };
+    auto spectral = [&](const V* row, uint32_t key) {
+#pragma unroll
+        for (int u = 0; u < E; ++u)
+            v[u] = fmul_spec<L>(v[u], row[tid + u * T], key + uint32_t(tid + u * T), u == 0 || u == E - 1);
+    };
+    auto spectral_ldg = [&](const V* __restrict__ row, uint32_t key) {
+#pragma unroll
+        for (int u = 0; u < E; ++u)
+            v[u] = fmul_spec<L>(v[u], __ldg(row + tid + u * T), key + uint32_t(tid + u * T), u == 0 || u == E - 1);
+    };
+    // v <- IFFT[ between . FFT v ]. ONE_TRANSFORM: one copy of the transform, the inverse as the forward
+    // transform of the conjugate, conjugated: less code to fetch against two sign flips per point.
+    // Measured with one copy / with two, FP64: 2048^2 6.73 / 7.09 ms, 1024^2 7.48 / 7.51, 3-D grids of 64
+    // to 256 points 2.74 / 2.66. FP32 passes keep both directions: 2048^2 13.2 / 12.5 ms, and the low parts
+    // of their split constants round differently in the conjugate (the sweep of 256^2 to 1024^2 members
+    // would gain 3%).
+    auto sandwich = [&](auto between) {
+        if constexpr (ONE_TRANSFORM) {
+#pragma unroll 1
+            for (int turn = 0; turn < 2; ++turn) {
+                fft_line_stages<L, E, -1, 0, TWS>(v, tid, line, tw, lsync);
+                if (turn == 0) between();
+                conjugate();
+            }
+        } else {
+            fft_line_stages<L, E, -1, 0, TWS>(v, tid, line, tw, lsync);
+            between();
+            fft_line_stages<L, E, +1, 0, TWS>(v, tid, line, tw, lsync);
+        }
+    };
 
-    if constexpr (MODE == PM_FFT_INV || MODE == PM_ROUNDTRIP) {
-        fft_line_stages<L, E, +1, 0, TWS>(v, tid, line, tw, lsync);
-    } else if constexpr (MODE != PM_DOUBLE) {
-        fft_line_stages<L, E, -1, 0, TWS>(v, tid, line, tw, lsync);
-    }
-
+    // A pass loops over one copy of the factors and reductions, at the places before, between and after
+    // its sandwiches. A launch finds the instruction caches cold: with a copy per place, 64 KB of code in
+    // the FP64 1024-point two-sandwich pass (30 KB now), its first transforms took 3,500 cycles each more
+    // than the second ones of the same launch.
     bool store_out = false;  // write v back to psi at the end
     if constexpr (MODE == PM_FFT_FWD || MODE == PM_FFT_INV) {
+        fft_line_stages<L, E, MODE == PM_FFT_FWD ? -1 : +1, 0, TWS>(v, tid, line, tw, lsync);
 #pragma unroll
         for (int u = 0; u < E; ++u) v[u] = cscale(v[u], a.scale);
         store_out = true;
     } else if constexpr (MODE == PM_ROUNDTRIP) {
+        fft_line_stages<L, E, +1, 0, TWS>(v, tid, line, tw, lsync);
 #pragma unroll
         for (int u = 0; u < E; ++u) v[u] = cscale(v[u], a.scale);
-        if (active)
-            apply_factors<R, E, T, true>(v, tid, base, lbase, a.mid_real, a.mid_cplx, a.mid_ax_cplx, a.mid_ax_real,
-                                         a.axis, a.dim, a.shift, a.nmask, nullptr, key0 ^ 0x2545f491u);
-        if (HAS_RED && a.red.n) {
-            if (active)
-                accumulate_line<R, E, T>(a.red, acc, v, a.partner, base, log2S, lbase, tid, a.axis, a.shift, a.nmask);
-            finish_red<NT>(a.red, acc, unsigned(g), ngroups);
-        }
+        if (active)  // a 1-D axis: no other axes
+            apply_tables<R, E, T, true>(v, tid, lbase, a.mid_real, a.mid_cplx, a.mid_ax_cplx[0], a.mid_ax_real[0],
+                                        false, V{}, false, R(1), key0 ^ 0x2545f491u);
+        if (HAS_RED && a.red.n) reduce();
         fft_line_stages<L, E, -1, 0, TWS>(v, tid, line, tw, lsync);
         store_out = true;
     } else if constexpr (MODE == PM_SPECRED) {
-        if (active) accumulate_line<R, E, T>(a.red, acc, v, a.partner, base, log2S, lbase, tid, a.axis, a.shift, a.nmask);
-    } else if constexpr (MODE == PM_DOUBLE) {
-        // The two sandwiches along the same axis as two turns of one loop, the r-space factor (and
-        // the reductions of a step boundary) after the first: the code of each transform direction
-        // exists once, so that the pass fits the instruction cache of the SM. The reducing variant
-        // (one pass per step) is unrolled: its accumulators would otherwise stay live in the loop.
-        constexpr int TURNS_UNROLLED = HAS_RED ? 2 : 1;
-#pragma unroll TURNS_UNROLLED
-        for (int half = 0; half < 2; ++half) {
-            fft_line_stages<L, E, -1, 0, TWS>(v, tid, line, tw, lsync);
-            const V* __restrict__ sp = half ? a.spec2 : (a.spec ? a.spec + (a.spec_full ? lbase : 0ll) : nullptr);
-            if (sp) {
-                const uint32_t kh = key0 + uint32_t(half * L);
-                if (SH::SPEC_SMEM && (half || spec_row)) {
-                    const V* sps = spec_s + (half ? L : 0);
+        fft_line_stages<L, E, -1, 0, TWS>(v, tid, line, tw, lsync);
+        reduce();
+    } else if constexpr (MODE == PM_APPLY) {
+        sandwich([&] {
+            if (a.spec) spectral_ldg(a.spec, key0);
+        });
+        if (active) {
+            // a branch-free loop per term, so that its reads go out together
+            auto flat_at = [&](int u) { return base + ((long long)(tid + u * T) << log2S); };
+            if (a.apply_vtab) {
 #pragma unroll
-                    for (int u = 0; u < E; ++u)
-                        v[u] = fmul_spec<L>(v[u], sps[tid + u * T], kh + uint32_t(tid + u * T), u == 0 || u == E - 1);
-                } else {
-#pragma unroll
-                    for (int u = 0; u < E; ++u)
-                        v[u] = fmul_spec<L>(v[u], __ldg(sp + tid + u * T), kh + uint32_t(tid + u * T),
-                                            u == 0 || u == E - 1);
-                }
+                for (int u = 0; u < E; ++u)
+                    v[u] = cadd(v[u], cscale(a.psi[flat_at(u)], R(__ldg(a.apply_vtab + flat_at(u)))));
             }
-            fft_line_stages<L, E, +1, 0, TWS>(v, tid, line, tw, lsync);
-            if (half == 0) {
-                if (active) {
-                    apply_factors<R, E, T>(v, tid, base, lbase, a.mid_real, a.mid_cplx, a.mid_ax_cplx, a.mid_ax_real,
-                                           a.axis, a.dim, a.shift, a.nmask, nullptr, key0 ^ 0x2545f491u);
-                    // a step boundary inside the pass: observables of the state between the two steps
-                    if (RED_MID && a.red.n)
-                        accumulate_line<R, E, T>(a.red, acc, v, a.partner, base, log2S, lbase, tid, a.axis, a.shift,
-                                                 a.nmask);
-                }
-                // finish those reductions here, so that no accumulator stays live through the second sandwich
-                if constexpr (HAS_RED) {
-                    if (RED_MID && a.red.n) finish_red<NT>(a.red, acc, unsigned(g), ngroups);
-                    // zero again whichever branch ran (the end reductions start from zero either way):
-                    // the compiler then holds no accumulator across the second sandwich
+            if (a.apply_acc) {
+                const V* __restrict__ sum = a.dst;
 #pragma unroll
-                    for (int k = 0; k < MAX_RED; ++k) acc[k] = 0.0;
-                }
+                for (int u = 0; u < E; ++u) v[u] = cadd(v[u], sum[flat_at(u)]);
+            }
+            if (a.dst) {
+#pragma unroll
+                for (int u = 0; u < E; ++u) a.dst[flat_at(u)] = v[u];
             }
         }
-        if (active) {
-            if (a.epi_real || a.epi_cplx || !a.ax_in_prologue)
-                apply_factors<R, E, T>(v, tid, base, lbase, a.epi_real, a.epi_cplx, a.ax_in_prologue ? nullptr : a.ax_cplx,
-                                       a.ax_real, a.axis, a.dim, a.shift, a.nmask, nullptr, key0 ^ 0x68e31da4u);
-            else
-                apply_factors<R, E, T>(v, tid, base, lbase, nullptr, nullptr, nullptr, a.ax_real, a.axis, a.dim,
-                                       a.shift, a.nmask, nullptr, key0 ^ 0x68e31da4u);
-            // the end of a chain of 1-D sandwich pairs: reductions of the final state
-            if (RED_END && a.red.n)
-                accumulate_line<R, E, T>(a.red, acc, v, a.partner, base, log2S, lbase, tid, a.axis, a.shift, a.nmask);
+        if (a.red.n) reduce();
+    } else {
+        // PROPAGATE: one sandwich or two; factors and reductions before the first, between them and after
+        // the last
+#pragma unroll 1
+        for (int half = 0;; ++half) {
+            const int place = half == 0 ? 0 : (half == a.sandwiches ? 2 : 1);
+            if (active && (a.points >> place & 1)) {
+                V lf = fone<V>();
+                R lr = R(1);
+                bool use_lf = false, use_lr = false;
+                const V* pc = nullptr;  // of the pass axis
+                const R* pr = nullptr;
+#pragma unroll
+                for (int k = 0; k < MAX_DIM; ++k) {
+                    if (k >= a.dim) break;  // the grid's axes only (a 2-D pass runs two turns of the six)
+                    const V* c = place == 1 ? a.mid_ax_cplx[k]
+                                            : ((place == 0) == (a.ax_in_prologue != 0) ? a.ax_cplx[k] : nullptr);
+                    const R* r = place == 1 ? a.mid_ax_real[k] : (place == 2 ? a.ax_real[k] : nullptr);
+                    if (k == a.axis) {
+                        pc = c;
+                        pr = r;
+                        continue;
+                    }
+                    const long long ik = (base >> a.shift[k]) & a.nmask[k];
+                    if (c) { lf = fcompose(lf, c[ik]); use_lf = true; }
+                    if (r) { lr *= r[ik]; use_lr = true; }
+                }
+                if (place == 0 && a.pro_scale_dev) { lr *= R(*a.pro_scale_dev); use_lr = true; }
+                apply_tables<R, E, T>(v, tid, lbase,
+                                      place == 0 ? a.pro_real : (place == 1 ? a.mid_real : a.epi_real),
+                                      place == 0 ? a.pro_cplx : (place == 1 ? a.mid_cplx : a.epi_cplx), pc, pr,
+                                      use_lf, lf, use_lr, lr,
+                                      key0 ^ (place == 0 ? 0x51ed270bu : (place == 1 ? 0x2545f491u : 0x68e31da4u)));
+            }
+            if (HAS_RED && a.red.n && place == (a.red_at_mid ? 1 : 2)) reduce();
+            if (place == 2) break;
+            sandwich([&] {
+                const V* __restrict__ sp = half ? a.spec2 : (a.spec ? a.spec + (a.spec_full ? lbase : 0ll) : nullptr);
+                const uint32_t kh = key0 + uint32_t(half * L);
+                if constexpr (SH::SPEC_SMEM) {  // host: never with spec_full
+                    if (sp) spectral(spec_s + half * L, kh);
+                } else {
+                    if (sp) spectral_ldg(sp, kh);
+                }
+            });
         }
         store_out = true;
-    } else {
-        // SANDWICH / APPLY: spectral multiply, inverse transform
-        if (a.spec) {
-            const V* __restrict__ sp = a.spec + (a.spec_full ? lbase : 0ll);
-            if (SH::SPEC_SMEM && MODE == PM_SANDWICH && spec_row) {
-#pragma unroll
-                for (int u = 0; u < E; ++u)
-                    v[u] = fmul_spec<L>(v[u], spec_s[tid + u * T], key0 + uint32_t(tid + u * T), u == 0 || u == E - 1);
-            } else {
-#pragma unroll
-                for (int u = 0; u < E; ++u)
-                    v[u] = fmul_spec<L>(v[u], __ldg(sp + tid + u * T), key0 + uint32_t(tid + u * T),
-                                        u == 0 || u == E - 1);
-            }
-        }
-        fft_line_stages<L, E, +1, 0, TWS>(v, tid, line, tw, lsync);
-        if (active) {
-            if constexpr (PROPAGATE) {
-                if (a.epi_real || a.epi_cplx || !a.ax_in_prologue)
-                    apply_factors<R, E, T>(v, tid, base, lbase, a.epi_real, a.epi_cplx,
-                                           a.ax_in_prologue ? nullptr : a.ax_cplx, a.ax_real, a.axis, a.dim, a.shift,
-                                           a.nmask, nullptr, key0 ^ 0x68e31da4u);
-                else
-                    apply_factors<R, E, T>(v, tid, base, lbase, nullptr, nullptr, nullptr, a.ax_real, a.axis, a.dim,
-                                           a.shift, a.nmask, nullptr, key0 ^ 0x68e31da4u);
-                if (HAS_RED && a.red.n && !a.red_at_mid)
-                    accumulate_line<R, E, T>(a.red, acc, v, a.partner, base, log2S, lbase, tid, a.axis, a.shift, a.nmask);
-            } else {  // PM_APPLY: a branch-free loop per term, so that its reads go out together
-                auto flat_at = [&](int u) { return base + ((long long)(tid + u * T) << log2S); };
-                if (a.apply_vtab) {
-#pragma unroll
-                    for (int u = 0; u < E; ++u)
-                        v[u] = cadd(v[u], cscale(a.psi[flat_at(u)], R(__ldg(a.apply_vtab + flat_at(u)))));
-                }
-                if (a.apply_acc) {
-                    const V* __restrict__ sum = a.dst;
-#pragma unroll
-                    for (int u = 0; u < E; ++u) v[u] = cadd(v[u], sum[flat_at(u)]);
-                }
-                if (a.red.n)
-                    accumulate_line<R, E, T>(a.red, acc, v, a.partner, base, log2S, lbase, tid, a.axis, a.shift, a.nmask);
-                if (a.dst) {
-#pragma unroll
-                    for (int u = 0; u < E; ++u) a.dst[base + ((long long)(tid + u * T) << log2S)] = v[u];
-                }
-            }
-        }
-        store_out = PROPAGATE;
     }
 
     if (store_out) {
@@ -849,9 +843,6 @@ __device__ __forceinline__ void pass_group(const PassArgs<R>& a, long long g, un
             for (int u = 0; u < E; ++u) out[base + tid + u * T] = v[u];
         }
     }
-    if constexpr (HAS_RED)
-        if (MODE == PM_SPECRED || (a.red.n && MODE != PM_ROUNDTRIP && (MODE == PM_DOUBLE ? RED_END : !a.red_at_mid)))
-            finish_red<NT>(a.red, acc, unsigned(g), ngroups);
 }
 
 template <typename R, int L, int SK, int KMODE, int VAR = 0>

@@ -21,10 +21,7 @@ template <typename R, int L, int VAR> static PassKernelInfo variant_info(int sk,
 #define QND_PICKV(M) QND_SK(R, L, M, VAR)
         switch (mode) {
         case PM_SANDWICH: fn = QND_PICKV(PM_SANDWICH); break;
-        case PM_DOUBLE: fn = QND_PICKV(PM_DOUBLE); break;
         case PM_SANDWICH_RED: fn = QND_PICKV(PM_SANDWICH_RED); break;
-        case PM_DOUBLE_RED: fn = QND_PICKV(PM_DOUBLE_RED); break;
-        case PM_DOUBLE_RED_END: fn = QND_PICKV(PM_DOUBLE_RED_END); break;
         default: fn = nullptr;
         }
 #undef QND_PICKV
@@ -46,12 +43,9 @@ template <typename R, int L> PassKernelInfo pass_kernel_info(bool strided, int m
     case PM_FFT_INV: fn = QND_PICK(PM_FFT_INV); break;
     case PM_SPECRED: fn = QND_PICK(PM_SPECRED); break;
     case PM_APPLY: fn = QND_PICK(PM_APPLY); break;
-    case PM_DOUBLE: fn = QND_PICK(PM_DOUBLE); break;
     case PM_ROUNDTRIP: fn = QND_PICK(PM_ROUNDTRIP); break;
     case PM_ROUNDTRIP_RED: fn = QND_PICK(PM_ROUNDTRIP_RED); break;
     case PM_SANDWICH_RED: fn = QND_PICK(PM_SANDWICH_RED); break;
-    case PM_DOUBLE_RED: fn = QND_PICK(PM_DOUBLE_RED); break;
-    case PM_DOUBLE_RED_END: fn = QND_PICK(PM_DOUBLE_RED_END); break;
     default: fn = nullptr;
     }
 #undef QND_PICK

@@ -49,9 +49,6 @@ __device__ __forceinline__ void sweep_dispatch_mode(const SweepSlot& sl, long lo
     switch (sl.kmode) {
     case PM_SANDWICH: sweep_run<R, L, S, PM_SANDWICH>(sl, g, smem); break;
     case PM_SANDWICH_RED: sweep_run<R, L, S, PM_SANDWICH_RED>(sl, g, smem); break;
-    case PM_DOUBLE: sweep_run<R, L, S, PM_DOUBLE>(sl, g, smem); break;
-    case PM_DOUBLE_RED: sweep_run<R, L, S, PM_DOUBLE_RED>(sl, g, smem); break;
-    case PM_DOUBLE_RED_END: sweep_run<R, L, S, PM_DOUBLE_RED_END>(sl, g, smem); break;
     default: break;  // the host records only these modes
     }
 }
@@ -167,7 +164,7 @@ template <typename R> cudaError_t launch_sweep(const SweepArgs& sa, cudaStream_t
     return cudaLaunchKernelExC(&lc, fn, args);
 }
 
-// one precision per compilation (-DQND_SWEEP_FP64=1 or 0): the kernel holds 32 pass bodies
+// one precision per compilation (-DQND_SWEEP_FP64=1 or 0): the kernel holds 16 pass bodies
 #if QND_SWEEP_FP64
 template cudaError_t launch_sweep<double>(const SweepArgs&, cudaStream_t, int, int*);
 #else
