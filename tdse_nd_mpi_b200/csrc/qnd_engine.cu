@@ -556,6 +556,7 @@ struct PassSpec {
     const void* ax_cplx[MAX_DIM] = {};
     const void* ax_real[MAX_DIM] = {};
     int ax_in_prologue = 0;
+    int from_p = 0, to_p = 0;    // see PassArgs
     double scale = 1.0;
     int apply_acc = 0;
     const double* apply_vtab = nullptr;
@@ -629,6 +630,9 @@ template <typename R> static void fill_args(qnd_ctx* c, const PassSpec& ps, Pass
     }
     a.ax_in_prologue = ps.ax_in_prologue;
     a.sandwiches = ps.mode == PM_DOUBLE ? 2 : 1;
+    a.from_p = ps.from_p;
+    a.to_p = ps.to_p;
+    a.p_scale = R(std::sqrt(double(c->nr[ps.axis])));
     bool ax = false, axr = false, mid = a.mid_real || a.mid_cplx;
     for (int k = 0; k < MAX_DIM; ++k) {
         ax = ax || a.ax_cplx[k];
@@ -857,7 +861,7 @@ static void load_shape_table() {
 
 static int shape_choice(qnd_ctx* c, const PassSpec& ps, int L, int log2S) {
     const int mode = ps.mode, kmode = pass_kernel_mode(mode, ps.red.n > 0);
-    if (ps.vL || (mode != PM_SANDWICH && mode != PM_DOUBLE) || L < 256 || L > 2048) return 0;
+    if (ps.vL || ps.from_p || ps.to_p || (mode != PM_SANDWICH && mode != PM_DOUBLE) || L < 256 || L > 2048) return 0;
     const bool strided = log2S > 0;
     if (const char* f = std::getenv("QND_SHAPE")) {
         const int v = std::atoi(f);
@@ -969,7 +973,7 @@ static void launch_pass(qnd_ctx* c, const PassSpec& ps) {
     const bool strided = log2S > 0;
     // passes that reduce run the instantiation that carries the reduction code; the others keep its
     // registers for the transform
-    const int kmode = pass_kernel_mode(ps.mode, ps.red.n > 0);
+    const int kmode = pass_kernel_mode(ps.mode, ps.red.n > 0, ps.from_p || ps.to_p);
     // the shape variant: the default while recording (the sweep kernel holds the default shapes)
     const int var = c->recorder ? 0 : (ps.force_shape >= 0 ? ps.force_shape : shape_choice(c, ps, L, log2S));
     const PassKernelInfo info = lookup_pass(c->fp64, L, strided, kmode, var);
@@ -1871,9 +1875,21 @@ static void run_chain1d(qnd_ctx* c, void* psi, const std::vector<ChainK>& K, con
 // in 2-D (2 NK + 1 in 3-D) instead of d NK; in 1-D the sandwiches pair up two per pass, and a
 // factor between pairs moves into the next pass's prologue (1-D chains carry no mask or
 // reductions between sandwiches).
+// from_p / to_p: psi is in the unitary momentum representation before K_0 / after K_{NK-1} (chain_ends_in_p
+// says where; pre and post are then empty): the passes of those sandwiches leave out the transform that
+// the change of representation would undo, which saves its d passes.
+static bool chain_ends_in_p(const qnd_ctx* c) {
+    if (c->dim < 2 || c->recorder) return false;
+    for (int j = 0; j < c->dim; ++j)
+        if (c->lax[j].on) return false;
+    return true;
+}
+
 static void run_chain(qnd_ctx* c, void* psi, const std::vector<ChainK>& K, const std::vector<ChainMid>& M,
-                      const Factor& pre, int64_t pre_lst, const double* pre_scale, const ChainMid& post) {
+                      const Factor& pre, int64_t pre_lst, const double* pre_scale, const ChainMid& post,
+                      bool from_p = false, bool to_p = false) {
     const int d = c->dim;
+    if ((from_p || to_p) && !chain_ends_in_p(c)) QND_FAIL(QND_EINVAL, "internal: a chain with ends in momentum space");
     const int64_t NK = int64_t(K.size());
     if (NK == 0 || int64_t(M.size()) != NK - 1) QND_FAIL(QND_EINVAL, "internal: malformed sandwich chain");
     if (chain1d(c)) {
@@ -1961,6 +1977,8 @@ static void run_chain(qnd_ctx* c, void* psi, const std::vector<ChainK>& K, const
             ps.axis = ax;
             ps.psi = psi;
             ps.spec = chain_spec(c, K[i], ax);
+            ps.from_p = from_p && i == 0;
+            ps.to_p = to_p && i + 1 == NK;
             if (i == 0 && q == 0) {
                 set_factor(c, pre, ax, pre_lst, &ps.pro_real, &ps.pro_cplx, ps.ax_cplx);
                 if (pre.laser_ia >= 0) ps.ax_in_prologue = 1;
@@ -1977,6 +1995,7 @@ static void run_chain(qnd_ctx* c, void* psi, const std::vector<ChainK>& K, const
                     ps.red_at_mid = 1;
                 }
                 ps.spec2 = chain_spec(c, K[i + 1], ax);
+                ps.to_p = to_p && i + 2 == NK;
             }
             if (q == d - 1 && i + 1 == NK) finish(ps);
             launch_pass(c, ps);
@@ -2057,7 +2076,9 @@ static void imag_chain1d(qnd_ctx* c, void* psi, int64_t n, const ChainGs& gs) {
 // rewritten in r-space): per step K(a_0) V(h_0) K(a_1 + a_2) V(h_1) ... V(h_{s-1}) K(a_{2s-1}); after
 // each step the step mask and the reductions red_fn(k, .) (of psi(t_{k+1})). A step boundary with
 // nothing on it merges K(a_{2s-1}) with the next step's K(a_0).
-static void length_steps(qnd_ctx* c, void* psi, int64_t lst0, int64_t n, const RedFn& red_fn, bool masked) {
+// from_p / to_p: see run_chain (no mask or reductions then).
+static void length_steps(qnd_ctx* c, void* psi, int64_t lst0, int64_t n, const RedFn& red_fn, bool masked,
+                         bool from_p = false, bool to_p = false) {
     if (n <= 0) return;
     if (c->dim == 1 && !c->long1d && !chain1d(c) && n > 1 && (masked || red_fn)) {
         // 1-D chains carry boundary work only at their end
@@ -2113,7 +2134,7 @@ static void length_steps(qnd_ctx* c, void* psi, int64_t lst0, int64_t n, const R
     post.lst = lst0 + n - 1;
     post.mask = masked;
     post.red = reductions(n - 1, false);
-    run_chain(c, psi, K, M, Factor{}, lst0, nullptr, post);
+    run_chain(c, psi, K, M, Factor{}, lst0, nullptr, post, from_p, to_p);
 }
 
 // Velocity-gauge steps lst0 .. lst0+n-1 in r-space (integrators.c:201-232); between steps the
@@ -3192,14 +3213,17 @@ int qnd_step_length(qnd_ctx* ctx, void* psi_p_dev, const double* E_host, int64_t
     if (nsteps <= 0) return QND_OK;
     QND_NEED(E_host);
     set_device(ctx);
-    unitary_fft(ctx, psi_p_dev, false);
+    // grids of several dimensions: the chain's ends take the changes of representation in; otherwise they
+    // are passes of their own
+    const bool ends = chain_ends_in_p(ctx);
+    if (!ends) unitary_fft(ctx, psi_p_dev, false);
     const int64_t chunk = chunk_steps(ctx);
     for (int64_t c0 = 0; c0 < nsteps; c0 += chunk) {
         const int64_t ch = std::min(chunk, nsteps - c0);
         upload_field_chunk(ctx, E_host + size_t(c0) * ctx->s * ctx->dim, ch, false);
-        length_steps(ctx, psi_p_dev, 0, ch, RedFn(), false);
+        length_steps(ctx, psi_p_dev, 0, ch, RedFn(), false, ends && c0 == 0, ends && c0 + ch == nsteps);
     }
-    unitary_fft(ctx, psi_p_dev, true);
+    if (!ends) unitary_fft(ctx, psi_p_dev, true);
     QND_CK(cudaGetLastError());
     check_finite(ctx, psi_p_dev, "qnd_step_length");
     QND_API_END

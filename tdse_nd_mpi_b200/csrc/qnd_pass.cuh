@@ -53,18 +53,21 @@ enum : int {
     PM_ROUNDTRIP = 6,
     PM_SANDWICH_RED = 7,  // with fused reductions: separate instantiations, so that the passes without them
     PM_ROUNDTRIP_RED = 8, // (most of a chain) keep their registers for the transform
-    PM_NMODES = 9
+    PM_SANDWICH_P = 9,    // the passes at a chain's ends in the momentum representation (PassArgs from_p, to_p):
+                          // with their tests in the kernels of every pass those ran 2% slower
+    PM_NMODES = 10
 };
 // The transform structure of a kernel's mode (the reducing variants share their base mode's), whether the
 // mode can carry reductions at all, and the kernel mode of a pass.
 __host__ __device__ constexpr int pass_base_mode(int m) {
-    return m == PM_SANDWICH_RED ? PM_SANDWICH : (m == PM_ROUNDTRIP_RED ? PM_ROUNDTRIP : m);
+    return m == PM_SANDWICH_RED || m == PM_SANDWICH_P ? PM_SANDWICH : (m == PM_ROUNDTRIP_RED ? PM_ROUNDTRIP : m);
 }
 __host__ __device__ constexpr bool pass_mode_reduces(int m) {
     return m == PM_SANDWICH_RED || m == PM_ROUNDTRIP_RED || m == PM_SPECRED || m == PM_APPLY;
 }
-__host__ __device__ constexpr int pass_kernel_mode(int m, bool reduces) {
-    return (m == PM_SANDWICH || m == PM_DOUBLE) ? (reduces ? PM_SANDWICH_RED : PM_SANDWICH)
+__host__ __device__ constexpr int pass_kernel_mode(int m, bool reduces, bool ends_in_p = false) {
+    return ends_in_p ? PM_SANDWICH_P
+           : (m == PM_SANDWICH || m == PM_DOUBLE) ? (reduces ? PM_SANDWICH_RED : PM_SANDWICH)
            : m == PM_ROUNDTRIP ? (reduces ? PM_ROUNDTRIP_RED : PM_ROUNDTRIP) : m;
 }
 // |v|^2 w, Re(conj(partner) v) w, or (element-wise grid reductions only) Im(conj(partner) v) w and
@@ -114,6 +117,10 @@ template <typename R> struct PassArgs {
     const R* mid_ax_real[MAX_DIM];  // PM_DOUBLE: per-axis real factors between the sandwiches (step mask)
     int red_at_mid;                 // PM_DOUBLE: reduce the state between the sandwiches, not at the end
     int sandwiches;                 // of a propagating pass: 1 or 2
+    // a pass at the end of a chain in the momentum representation: the first sandwich without its forward
+    // transform, the last one without its inverse; each takes the place of two transforms and a scaling
+    int from_p, to_p;
+    R p_scale;                      // with either: sqrt(L) (the tables hold 1/L, the representation 1/sqrt(L))
     int points;                     // bits of the places with factors: 1 before, 2 between the sandwiches, 4 after
     const R* epi_real;
     const V* epi_cplx;
@@ -530,7 +537,7 @@ __device__ __forceinline__ void pass_group(const PassArgs<R>& a, long long g, un
     constexpr bool TMA = SK == 2;
     constexpr int MODE = pass_base_mode(KMODE);
     constexpr bool HAS_RED = pass_mode_reduces(KMODE);
-    constexpr bool PROPAGATE = MODE == PM_SANDWICH;
+    constexpr bool PROPAGATE = MODE == PM_SANDWICH, ENDS = KMODE == PM_SANDWICH_P;
     constexpr bool ONE_TRANSFORM = sizeof(R) == 8 && L >= 1024;  // see the sandwich below
     using V = cplx_t<R>;
     using SH = PassShape<R, L, VAR>;
@@ -687,18 +694,20 @@ __device__ __forceinline__ void pass_group(const PassArgs<R>& a, long long g, un
     // to 256 points 2.74 / 2.66. FP32 passes keep both directions: 2048^2 13.2 / 12.5 ms, and the low parts
     // of their split constants round differently in the conjugate (the sweep of 256^2 to 1024^2 members
     // would gain 3%).
-    auto sandwich = [&](auto between) {
+    // fwd / inv: whether the transforms run (PassArgs from_p, to_p).
+    auto sandwich = [&](bool fwd, bool inv, auto between) {
         if constexpr (ONE_TRANSFORM) {
 #pragma unroll 1
             for (int turn = 0; turn < 2; ++turn) {
-                fft_line_stages<L, E, -1, 0, TWS>(v, tid, line, tw, lsync);
+                if (turn || fwd) fft_line_stages<L, E, -1, 0, TWS>(v, tid, line, tw, lsync);
                 if (turn == 0) between();
+                if (!inv) break;
                 conjugate();
             }
         } else {
-            fft_line_stages<L, E, -1, 0, TWS>(v, tid, line, tw, lsync);
+            if (fwd) fft_line_stages<L, E, -1, 0, TWS>(v, tid, line, tw, lsync);
             between();
-            fft_line_stages<L, E, +1, 0, TWS>(v, tid, line, tw, lsync);
+            if (inv) fft_line_stages<L, E, +1, 0, TWS>(v, tid, line, tw, lsync);
         }
     };
 
@@ -726,7 +735,7 @@ __device__ __forceinline__ void pass_group(const PassArgs<R>& a, long long g, un
         fft_line_stages<L, E, -1, 0, TWS>(v, tid, line, tw, lsync);
         reduce();
     } else if constexpr (MODE == PM_APPLY) {
-        sandwich([&] {
+        sandwich(true, true, [&] {
             if (a.spec) spectral_ldg(a.spec, key0);
         });
         if (active) {
@@ -784,13 +793,19 @@ __device__ __forceinline__ void pass_group(const PassArgs<R>& a, long long g, un
             }
             if (HAS_RED && a.red.n && place == (a.red_at_mid ? 1 : 2)) reduce();
             if (place == 2) break;
-            sandwich([&] {
+            const bool fwd = !ENDS || half > 0 || !a.from_p, inv = !ENDS || half + 1 < a.sandwiches || !a.to_p;
+            sandwich(fwd, inv, [&] {
                 const V* __restrict__ sp = half ? a.spec2 : (a.spec ? a.spec + (a.spec_full ? lbase : 0ll) : nullptr);
                 const uint32_t kh = key0 + uint32_t(half * L);
                 if constexpr (SH::SPEC_SMEM) {  // host: never with spec_full
                     if (sp) spectral(spec_s + half * L, kh);
                 } else {
                     if (sp) spectral_ldg(sp, kh);
+                }
+                if (!fwd || !inv) {
+                    const R sc = (fwd || inv) ? a.p_scale : a.p_scale * a.p_scale;
+#pragma unroll
+                    for (int u = 0; u < E; ++u) v[u] = cscale(v[u], sc);
                 }
             });
         }

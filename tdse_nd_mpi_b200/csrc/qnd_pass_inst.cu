@@ -46,6 +46,7 @@ template <typename R, int L> PassKernelInfo pass_kernel_info(bool strided, int m
     case PM_ROUNDTRIP: fn = QND_PICK(PM_ROUNDTRIP); break;
     case PM_ROUNDTRIP_RED: fn = QND_PICK(PM_ROUNDTRIP_RED); break;
     case PM_SANDWICH_RED: fn = QND_PICK(PM_SANDWICH_RED); break;
+    case PM_SANDWICH_P: fn = QND_PICK(PM_SANDWICH_P); break;
     default: fn = nullptr;
     }
 #undef QND_PICK
