@@ -16,7 +16,7 @@
 
 namespace qnd {
 
-// Sums of n (at most MAX_RED) accumulators over the CTA's T threads, to out[0..n) in shared memory,
+// Sums of n (at most MAX_RED) accumulators over the CTA's T threads (whole warps), to out[0..n) in shared memory,
 // visible to every thread on return. red: [T / 32][MAX_RED] shared scratch.
 template <int T> __device__ __forceinline__ void cta_sums(const double* acc, int n, double (*red)[MAX_RED], double* out) {
     const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
@@ -39,6 +39,7 @@ template <int T> __device__ __forceinline__ void cta_sums(const double* acc, int
 template <typename R, int L, int E> struct ChainShape {
     using P = FFTPlan<L, E>;
     static constexpr int T = L / E;
+    static constexpr int NT = T < 32 ? 32 : T;  // threads: a shorter line's lanes are repeated over one warp
     static constexpr int TW = ((sizeof(R) == 8 ? P::twb_size() : P::tw_size()) + 1) & ~1;
     static constexpr size_t SMEM = sizeof(cplx_t<R>) * (size_t(TW) + P::SMEM_LINE);
 };
@@ -92,14 +93,15 @@ __global__ void __launch_bounds__(L / E, 1) qnd_chain1d_kernel(const __grid_cons
         if (op.obs >= 0) {
 #pragma unroll 1
             for (int k = 0; k < a.red.n; ++k) {
-                const double s = warp_sum(line_sum<R, E, T>(red_sh.row[k], v, static_cast<const V*>(nullptr), 0, 0, 0, tid));
-                if ((tid & 31) == 0) red_sh.s[tid >> 5][k] = s;
+                const double own = line_sum<R, E, T>(red_sh.row[k], v, static_cast<const V*>(nullptr), 0, 0, 0, tid);
+                const double s = warp_sum(counts ? own : 0.0);
+                if ((t & 31) == 0) red_sh.s[t >> 5][k] = s;
             }
             __syncthreads();
-            if (tid < a.red.n) {
+            if (t < a.red.n) {
                 double s = 0.0;
-                for (int w = 0; w < T / 32; ++w) s += red_sh.s[w][tid];
-                a.red.out[op.obs + tid] = s * a.red.scale[tid];
+                for (int w = 0; w < NT / 32; ++w) s += red_sh.s[w][t];
+                a.red.out[op.obs + t] = s * a.red.scale[t];
             }
             __syncthreads();  // the warps' sums are read
         }
@@ -110,7 +112,7 @@ __global__ void __launch_bounds__(L / E, 1) qnd_chain1d_kernel(const __grid_cons
 #pragma unroll
                 for (int q = 0; q < MAX_RED / 2; ++q) {
                     acc[2 * q] = acc[2 * q + 1] = 0.0;
-                    if (k0 + q >= a.ngs) continue;
+                    if (k0 + q >= a.ngs || !counts) continue;
                     const V* __restrict__ s = a.states[k0 + q];
 #pragma unroll
                     for (int u = 0; u < E; ++u) {
@@ -120,8 +122,8 @@ __global__ void __launch_bounds__(L / E, 1) qnd_chain1d_kernel(const __grid_cons
                     }
                 }
                 const int n = 2 * (a.ngs - k0 < MAX_RED / 2 ? a.ngs - k0 : MAX_RED / 2);
-                cta_sums<T>(acc, n, red_s, sum_s);
-                if (tid < n) coef_s[2 * k0 + tid] = sum_s[tid] * a.dNr;
+                cta_sums<NT>(acc, n, red_s, sum_s);
+                if (t < n) coef_s[2 * k0 + t] = sum_s[t] * a.dNr;
                 __syncthreads();
             }
             for (int k = 0; k < a.ngs; ++k) {
@@ -137,11 +139,12 @@ __global__ void __launch_bounds__(L / E, 1) qnd_chain1d_kernel(const __grid_cons
             double acc[1] = {0.0};
 #pragma unroll
             for (int u = 0; u < E; ++u) acc[0] += double(v[u].x) * double(v[u].x) + double(v[u].y) * double(v[u].y);
-            cta_sums<T>(acc, 1, red_s, sum_s);
+            if (!counts) acc[0] = 0.0;
+            cta_sums<NT>(acc, 1, red_s, sum_s);
             const double n2 = sum_s[0] * a.dNr;
             double scale = 1.0;
             if (n2 < a.gs_tol || !(n2 == n2)) {
-                if (tid == 0) *a.gs_flag = 1;
+                if (t == 0) *a.gs_flag = 1;
             } else {
                 scale = 1.0 / sqrt(n2);
             }
@@ -156,14 +159,14 @@ __global__ void __launch_bounds__(L / E, 1) qnd_chain1d_kernel(const __grid_cons
 }
 
 template <typename R, int L> static cudaError_t launch_one(const Chain1dArgs<R>& a, cudaStream_t st) {
-    constexpr int E = chain1d_values(L);
+    constexpr int E = chain1d_values(L, sizeof(R) == 8);
     using SH = ChainShape<R, L, E>;
     auto* fn = &qnd_chain1d_kernel<R, L, E>;
     if constexpr (SH::SMEM > 48 * 1024) {
         const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(SH::SMEM));
         if (e != cudaSuccess) return e;
     }
-    fn<<<1, SH::T, SH::SMEM, st>>>(a);
+    fn<<<1, SH::NT, SH::SMEM, st>>>(a);
     return cudaGetLastError();
 }
 

@@ -196,10 +196,11 @@ struct qnd_ctx {
     DevBuf tune_buf;                            // scratch state of the staging autotuner
     DevBuf shape_buf;                           // scratch state of the shape autotuner (its own: the
                                                 // staging tuner frees tune_buf inside its launches)
+    DevBuf adjoint_buf;                         // workspace of the adjoint calls (adjoint_run)
     DevBuf finite_slot;                         // QND_CHECK_FINITE: the non-finite count
     std::map<std::tuple<const void*, int, int>, CUtensorMap> tmaps;  // strided-pass TMA views of states
 
-    // A 1-D axis longer than one pass handles: N = n1 n2 (64 to 4096 each) as a virtual
+    // A 1-D axis longer than one pass handles: N = n1 n2 (16 to 4096 each) as a virtual
     // n1 x n2 grid transformed in four steps (long_fft). tw_long[v]: the stage twiddles of the
     // length-n1 (v = 0) and length-n2 (v = 1) passes; twf_long / twc_long: the four-step twiddle
     // W_N^{k1 m} and its conjugate at slot k1 n2 + m; p_slot: the momentum of each k-space slot
@@ -2762,13 +2763,18 @@ static void build_long_axis_nd(qnd_ctx* c, int ax) {
 static void build_long_axis(qnd_ctx* c) {
     const int64_t N = c->nr[0];
     c->long1d = true;
-    // Two lengths of about the same size (the shorter one strided), 64 to 4096 points each: both virtual
-    // axes then have many lines to spread over the SMs (64 x 4096 gave the contiguous pass of 262144
-    // points 64 CTAs for 148 SMs, 29.6 us). From 2^16 to 2^18 points the contiguous axis takes 256 points,
-    // two radix-16 stages. us per FP64 BM4 step with observables: 2^17 as 512 x 256 101, as 256 x 512 108;
-    // 2^18 as 1024 x 256 117, as 512 x 512 122, as 256 x 1024 125; 2^19 as 512 x 1024 172, as 2048 x 256
-    // 181; 2^20 as 1024 x 1024 276, as 4096 x 256 477.
-    c->lg1 = c->lognr[0] >= 16 && c->lognr[0] <= 18 ? c->lognr[0] - 8 : c->lognr[0] / 2;
+    // FP64: two lengths of about the same size (the shorter one strided), 64 to 4096 points each: both
+    // virtual axes then have many lines to spread over the SMs (64 x 4096 gave the contiguous pass of
+    // 262144 points 64 CTAs for 148 SMs, 29.6 us). From 2^16 to 2^18 points the contiguous axis takes 256
+    // points, two radix-16 stages. us per BM4 step with observables: 2^17 as 512 x 256 101, as 256 x 512
+    // 108; 2^18 as 1024 x 256 117, as 512 x 512 122, as 256 x 1024 125; 2^19 as 512 x 1024 172, as
+    // 2048 x 256 181; 2^20 as 1024 x 1024 276, as 4096 x 256 477.
+    // FP32: the split also sets the rounding. 16 points strided up to 2^15 and 256 after (up to 4096
+    // contiguous) are the fastest splits whose errors against 64 bits stay those of n2 = 4096: after 16
+    // imaginary-time steps 8192 points are 2.5e-6 off as 16 x 512 and 4.0e-6 as 64 x 128, 131072 9.4e-6 as
+    // 32 x 4096, 6.9e-6 as 256 x 512 and 1.1e-5 as 512 x 256 (125, 78 and 80 us a step).
+    if (c->fp64) c->lg1 = c->lognr[0] >= 16 && c->lognr[0] <= 18 ? c->lognr[0] - 8 : c->lognr[0] / 2;
+    else c->lg1 = c->lognr[0] <= 15 ? 4 : std::max(8, c->lognr[0] - 12);
     c->lg2 = c->lognr[0] - c->lg1;
     c->n1 = int64_t(1) << c->lg1;
     c->n2 = int64_t(1) << c->lg2;
@@ -2875,7 +2881,7 @@ static void build_context(qnd_ctx* c, int dim, const int64_t* nr, const double* 
             build_twiddles(c, int(c->nr[j]), c->tw[j]);
         }
     }
-    if (dim == 1 && chain1d_length_ok(c->nr[0])) build_twiddles(c, int(c->nr[0]), c->tw_chain, chain1d_values(int(c->nr[0])));
+    if (dim == 1 && chain1d_length_ok(c->nr[0])) build_twiddles(c, int(c->nr[0]), c->tw_chain, chain1d_values(int(c->nr[0]), c->fp64));
     if (any_long) {
         // the scratch states of the emulated passes, allocated up front (not inside a graph capture)
         c->lax_perm.ensure(size_t(c->n) * c->elem());

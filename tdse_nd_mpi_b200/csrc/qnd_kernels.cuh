@@ -205,11 +205,13 @@ template <typename R> void launch_apply_combine(long long n, cplx_t<R>* dst, con
 // ---- 1-D grids of up to 4096 points: a chain of sandwiches in one launch (qnd_chain1d.cu)
 constexpr int CHAIN1D_OPS = 512;     // sandwiches per launch (longer chains take several launches)
 constexpr int CHAIN1D_TABLES = 24;   // distinct spectral / r-space tables per launch
-// Line lengths the chain kernel is built for, and its values per thread (whole warps on one line).
+// Line lengths the chain kernel is built for, and its values per thread.
+// FP32 keeps the pass kernels' 16 at every length, with them their stages and their roundings: with 8 (a
+// stage more, and twice the dithered factors) a 256-point run was twice as far from 64-bit results.
 // Measured with FP64, us per BM4 step with observables: 512 points 12.7 with 8 values (4: 16.6, 16: 19.1),
 // 1024 19.1 (16: 21.4), 2048 27.7 with 16 (8: 29.6), 4096 (imaginary time) 37 with 16 (8: 44).
 constexpr bool chain1d_length_ok(long long L) { return L >= 128 && L <= 4096 && (L & (L - 1)) == 0; }
-constexpr int chain1d_values(int L) { return L == 128 ? 4 : (L < 2048 ? 8 : 16); }
+constexpr int chain1d_values(int L, bool fp64) { return !fp64 ? 16 : (L == 128 ? 4 : (L < 2048 ? 8 : 16)); }
 // One sandwich and the point-wise work after it, in this order: factor `mid` with the laser phases and
 // the step mask, reductions into red.out + obs, Gram-Schmidt, factor `mid2`.
 struct Chain1dOp {
@@ -223,7 +225,8 @@ struct Chain1dOp {
 template <typename R> struct Chain1dArgs {
     using V = cplx_t<R>;
     V* psi;
-    const V* tw;          // stage twiddles for chain1d_values(L) values per thread
+    const V* src;         // where the state is read (psi, or another state that stays)
+    const V* tw;          // stage twiddles for chain1d_values values per thread
     const V* field;       // per-step field tables
     const V* spec[CHAIN1D_TABLES];
     const R* mid_real[CHAIN1D_TABLES];
