@@ -487,6 +487,47 @@ __global__ void __launch_bounds__(256) apply_combine_kernel(long long n, cplx_t<
     }
 }
 
+template <typename R>
+__global__ void __launch_bounds__(256) weight_state_kernel(long long n, cplx_t<R>* dst, const cplx_t<R>* psi,
+                                                           const double* w, double scale) {
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
+        dst[i] = cscale(psi[i], R(scale * w[i]));
+}
+
+// The product of two states once per point for the sums of all axes, four points on their way per thread
+// (bound by the two states' reads): 31 us -> 14 us at 128^3 FP64 against the general grid reduction,
+// which reads the partner for every accumulator and one point at a time.
+template <typename R>
+__global__ void __launch_bounds__(256) axis_im_reduce_kernel(const __grid_constant__ AxisImArgs args,
+                                                             const cplx_t<R>* __restrict__ a,
+                                                             const cplx_t<R>* __restrict__ b) {
+    double acc[MAX_RED];
+#pragma unroll
+    for (int k = 0; k < MAX_RED; ++k) acc[k] = 0.0;
+    const long long step = (long long)gridDim.x * blockDim.x;
+    for (long long i0 = (long long)blockIdx.x * blockDim.x + threadIdx.x; i0 < args.n; i0 += 4 * step) {
+        cplx_t<R> p[4], v[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const long long i = i0 + q * step;
+            p[q] = v[q] = cplx_t<R>{R(0), R(0)};
+            if (i < args.n) {
+                p[q] = a[i];
+                v[q] = b[i];
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const long long i = i0 + q * step;
+            const double val = double(p[q].x) * double(v[q].y) - double(p[q].y) * double(v[q].x);
+#pragma unroll
+            for (int j = 0; j < MAX_DIM; ++j)
+                if (j < args.dim) acc[j] += val * __ldg(args.red.wtab[j] + ((i >> args.shift[j]) & args.nmask[j]));
+        }
+    }
+    finish_red<256>(args.red, acc);
+}
+
 struct MaskArgs {
     int dim;
     int shift[MAX_DIM];
@@ -533,6 +574,14 @@ template <typename R> void launch_apply_masks(long long n, cplx_t<R>* psi, int d
     }
     apply_masks_kernel<R><<<elementwise_blocks(n), 256, 0, st>>>(n, psi, a);
 }
+template <typename R> void launch_weight_state(long long n, cplx_t<R>* dst, const cplx_t<R>* psi, const double* w,
+                                               double scale, cudaStream_t st) {
+    weight_state_kernel<R><<<elementwise_blocks(n), 256, 0, st>>>(n, dst, psi, w, scale);
+}
+template <typename R> void launch_axis_im_reduce(const AxisImArgs& args, const cplx_t<R>* a, const cplx_t<R>* b,
+                                                 cudaStream_t st, int nblocks) {
+    axis_im_reduce_kernel<R><<<nblocks, 256, 0, st>>>(args, a, b);
+}
 template <typename R> void launch_add_potential(long long n, cplx_t<R>* dst, const cplx_t<R>* src, const double* vtab,
                                                 cudaStream_t st) {
     add_potential_kernel<R><<<elementwise_blocks(n), 256, 0, st>>>(n, dst, src, vtab);
@@ -565,6 +614,9 @@ template <typename R> void launch_apply_combine(long long n, cplx_t<R>* dst, con
     template void launch_point_factors<R>(long long, cplx_t<R>*, const R*, const cplx_t<R>*, const cplx_t<R>*, \
                                           const LongArgs&, const R*, const double*, cudaStream_t);         \
     template void launch_add_potential<R>(long long, cplx_t<R>*, const cplx_t<R>*, const double*, cudaStream_t); \
+    template void launch_weight_state<R>(long long, cplx_t<R>*, const cplx_t<R>*, const double*, double,      \
+                                         cudaStream_t);                                                      \
+    template void launch_axis_im_reduce<R>(const AxisImArgs&, const cplx_t<R>*, const cplx_t<R>*, cudaStream_t, int); \
     template void launch_embed<R>(const EmbedArgs&, const double2*, cplx_t<R>*, cudaStream_t);                \
     template void launch_apply_masks<R>(long long, cplx_t<R>*, int, const int*, const long long*, const R* const*, \
                                         cudaStream_t);                                                      \

@@ -45,26 +45,30 @@ template <typename R, int L, int E> struct ChainShape {
 };
 
 template <typename R, int L, int E>
-__global__ void __launch_bounds__(L / E, 1) qnd_chain1d_kernel(const __grid_constant__ Chain1dArgs<R> a) {
+__global__ void __launch_bounds__(ChainShape<R, L, E>::NT, 1) qnd_chain1d_kernel(const __grid_constant__ Chain1dArgs<R> a) {
     using V = cplx_t<R>;
     using SH = ChainShape<R, L, E>;
-    constexpr int T = SH::T;
-    static_assert(T >= 32 && T % 32 == 0, "whole warps");
+    constexpr int T = SH::T, NT = SH::NT;
+    static_assert(T % 32 == 0 || 32 % T == 0, "whole warps, or lanes repeated over one");
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    __shared__ double red_s[T / 32][MAX_RED];
-    __shared__ RedShared<T> red_sh;
+    __shared__ double red_s[NT / 32][MAX_RED];
+    __shared__ RedShared<NT> red_sh;
     __shared__ double sum_s[MAX_RED];
     __shared__ double coef_s[2 * GS_MAXK];
     V* tw = reinterpret_cast<V*>(smem_raw);
     V* line = tw + SH::TW;
-    const int tid = threadIdx.x;
+    const int t = threadIdx.x;
+    // Lanes past T repeat the first ones' work on the same addresses with the same values; only the first
+    // T count in sums.
+    const int tid = t % T;
+    const bool counts = t < T;
     const LineSync<T> lsync{1};
 
-    for (int i = tid; i < (sizeof(R) == 8 ? SH::P::twb_size() : SH::P::tw_size()); i += T) tw[i] = a.tw[i];
+    for (int i = t; i < (sizeof(R) == 8 ? SH::P::twb_size() : SH::P::tw_size()); i += NT) tw[i] = a.tw[i];
     V v[E];
 #pragma unroll
-    for (int u = 0; u < E; ++u) v[u] = a.psi[tid + u * T];
-    load_red_rows<T>(a.red, 0, red_sh);
+    for (int u = 0; u < E; ++u) v[u] = a.src[tid + u * T];
+    load_red_rows<NT>(a.red, 0, red_sh);
     __syncthreads();  // twiddles and reductions visible
 
     // the point-wise factor `mid` (a full-grid table) with the laser phases at `laser`, the step mask

@@ -540,6 +540,7 @@ struct PassSpec {
     int axis = 0;
     int mode = PM_SANDWICH;
     void* psi = nullptr;
+    const void* src = nullptr;   // contiguous axes: read from here instead of psi
     void* dst = nullptr;
     const void* partner = nullptr;
     const void* pro_real = nullptr;
@@ -602,6 +603,7 @@ template <typename R> static void fill_args(qnd_ctx* c, const PassSpec& ps, Pass
     using V = cplx_t<R>;
     std::memset(&a, 0, sizeof a);
     a.psi = static_cast<V*>(ps.psi);
+    a.src = ps.src ? static_cast<const V*>(ps.src) : a.psi;
     a.dst = static_cast<V*>(ps.dst);
     a.axis = ps.axis;
     a.partner = static_cast<const V*>(ps.partner);
@@ -897,6 +899,7 @@ static int shape_choice(qnd_ctx* c, const PassSpec& ps, int L, int log2S) {
     t.mode = mode;
     t.red = RedDesc{};
     t.red_at_mid = 0;
+    t.src = nullptr;
     t.psi = c->shape_buf.p;
     const int64_t k0 = c->kernels_launched;
     cudaEvent_t e0, e1;
@@ -1780,7 +1783,7 @@ struct ChainGs {
 
 static void run_chain1d(qnd_ctx* c, void* psi, const std::vector<ChainK>& K, const std::vector<ChainMid>& M,
                         const Factor& pre, int64_t pre_lst, const double* pre_scale, const ChainMid& post,
-                        const ChainGs& gs = ChainGs()) {
+                        const ChainGs& gs = ChainGs(), const void* src = nullptr) {
     const int64_t NK = int64_t(K.size());
     auto run = [&](auto tag) {
         using R = decltype(tag);
@@ -1793,6 +1796,8 @@ static void run_chain1d(qnd_ctx* c, void* psi, const std::vector<ChainK>& K, con
         auto begin = [&]() {
             a = Chain1dArgs<R>{};
             a.psi = static_cast<V*>(psi);
+            a.src = src ? static_cast<const V*>(src) : a.psi;
+            src = nullptr;  // a later launch goes on from psi
             a.tw = c->tw_chain.as<V>();
             a.field = field;
             a.mask = c->mask_dev[0].as<R>();
@@ -1886,15 +1891,25 @@ static bool chain_ends_in_p(const qnd_ctx* c) {
     return true;
 }
 
+static void copy_state(qnd_ctx* c, void* dst, const void* src) {
+    QND_CK(cudaMemcpyAsync(dst, src, size_t(c->n) * c->elem(), cudaMemcpyDeviceToDevice, c->stream));
+}
+
 static void run_chain(qnd_ctx* c, void* psi, const std::vector<ChainK>& K, const std::vector<ChainMid>& M,
                       const Factor& pre, int64_t pre_lst, const double* pre_scale, const ChainMid& post,
-                      bool from_p = false, bool to_p = false) {
+                      bool from_p = false, bool to_p = false, const void* src = nullptr) {
     const int d = c->dim;
+    // src: the state the chain starts from, left as it is (null: psi). Its first pass, along the contiguous
+    // axis, reads it; where the chain starts otherwise it is copied.
+    if (src && !chain1d(c) && (c->long1d || c->recorder || c->lax[d - 1].on)) {
+        copy_state(c, psi, src);
+        src = nullptr;
+    }
     if ((from_p || to_p) && !chain_ends_in_p(c)) QND_FAIL(QND_EINVAL, "internal: a chain with ends in momentum space");
     const int64_t NK = int64_t(K.size());
     if (NK == 0 || int64_t(M.size()) != NK - 1) QND_FAIL(QND_EINVAL, "internal: malformed sandwich chain");
     if (chain1d(c)) {
-        run_chain1d(c, psi, K, M, pre, pre_lst, pre_scale, post);
+        run_chain1d(c, psi, K, M, pre, pre_lst, pre_scale, post, ChainGs(), src);
         return;
     }
     if (c->long1d) {
@@ -1945,6 +1960,7 @@ static void run_chain(qnd_ctx* c, void* psi, const std::vector<ChainK>& K, const
             PassSpec ps;
             ps.axis = 0;
             ps.psi = psi;
+            if (i == 0) ps.src = src;
             ps.spec = chain_spec(c, K[i], 0);
             if (i == 0) {
                 set_factor(c, pre, 0, pre_lst, &ps.pro_real, &ps.pro_cplx, ps.ax_cplx);
@@ -1981,6 +1997,7 @@ static void run_chain(qnd_ctx* c, void* psi, const std::vector<ChainK>& K, const
             ps.from_p = from_p && i == 0;
             ps.to_p = to_p && i + 1 == NK;
             if (i == 0 && q == 0) {
+                ps.src = src;
                 set_factor(c, pre, ax, pre_lst, &ps.pro_real, &ps.pro_cplx, ps.ax_cplx);
                 if (pre.laser_ia >= 0) ps.ax_in_prologue = 1;
                 ps.pro_scale = pre_scale;
@@ -2079,13 +2096,13 @@ static void imag_chain1d(qnd_ctx* c, void* psi, int64_t n, const ChainGs& gs) {
 // nothing on it merges K(a_{2s-1}) with the next step's K(a_0).
 // from_p / to_p: see run_chain (no mask or reductions then).
 static void length_steps(qnd_ctx* c, void* psi, int64_t lst0, int64_t n, const RedFn& red_fn, bool masked,
-                         bool from_p = false, bool to_p = false) {
+                         bool from_p = false, bool to_p = false, const void* src = nullptr) {
     if (n <= 0) return;
     if (c->dim == 1 && !c->long1d && !chain1d(c) && n > 1 && (masked || red_fn)) {
         // 1-D chains carry boundary work only at their end
         for (int64_t k = 0; k < n; ++k)
             length_steps(c, psi, lst0 + k, 1, red_fn ? RedFn([&](int64_t, int ax) { return red_fn(k, ax); }) : RedFn(),
-                         masked);
+                         masked, false, false, k == 0 ? src : nullptr);
         return;
     }
     const int s = c->s;
@@ -2135,7 +2152,7 @@ static void length_steps(qnd_ctx* c, void* psi, int64_t lst0, int64_t n, const R
     post.lst = lst0 + n - 1;
     post.mask = masked;
     post.red = reductions(n - 1, false);
-    run_chain(c, psi, K, M, Factor{}, lst0, nullptr, post, from_p, to_p);
+    run_chain(c, psi, K, M, Factor{}, lst0, nullptr, post, from_p, to_p, src);
 }
 
 // Velocity-gauge steps lst0 .. lst0+n-1 in r-space (integrators.c:201-232); between steps the
@@ -2143,7 +2160,7 @@ static void length_steps(qnd_ctx* c, void* psi, int64_t lst0, int64_t n, const R
 // last step only; on the grids of the chain kernel (chain1d), red_fn (in place of fin) and the mask
 // apply after every step.
 static void velocity_steps(qnd_ctx* c, void* psi, int64_t lst0, int64_t n, const RedDesc* fin, bool masked,
-                           const RedFn& red_fn = RedFn()) {
+                           const RedFn& red_fn = RedFn(), const void* src = nullptr) {
     if (n <= 0) return;
     const int s = c->s;
     std::vector<std::vector<RedDesc>> reds;
@@ -2187,7 +2204,7 @@ static void velocity_steps(qnd_ctx* c, void* psi, int64_t lst0, int64_t n, const
     post.lst = lst0 + n - 1;
     post.mask = masked;
     post.red = red_fn ? reductions(n - 1) : fin;
-    run_chain(c, psi, K, M, pre, lst0, nullptr, post);
+    run_chain(c, psi, K, M, pre, lst0, nullptr, post, false, false, src);
 }
 
 static void unitary_fft(qnd_ctx* c, void* psi, bool forward) {
@@ -2449,20 +2466,21 @@ static void apply_table(qnd_ctx* c, void* psi, const void* table) {
     QND_CK(cudaGetLastError());
 }
 
-static void copy_state(qnd_ctx* c, void* dst, const void* src) {
-    QND_CK(cudaMemcpyAsync(dst, src, size_t(c->n) * c->elem(), cudaMemcpyDeviceToDevice, c->stream));
-}
-
-// Steps k0 .. k0+n-1 of the run's field samples (host [nsteps][s][dim]) on an r-space psi.
-static void steps_span(qnd_ctx* c, void* psi, const double* F, int64_t k0, int64_t n, bool masked, bool velocity) {
+// Steps k0 .. k0+n-1 of the run's field samples (host [nsteps][s][dim]): psi <- steps of src.
+static void steps_span(qnd_ctx* c, void* psi, const void* src, const double* F, int64_t k0, int64_t n, bool masked,
+                       bool velocity) {
     const int64_t chunk = chunk_steps(c);
     for (int64_t q = 0; q < n; q += chunk) {
         const int64_t ch = std::min(chunk, n - q);
         upload_field_chunk(c, F + size_t(k0 + q) * c->s * c->dim, ch, velocity);
-        if (!velocity) length_steps(c, psi, 0, ch, RedFn(), masked);
-        else if (!masked) velocity_steps(c, psi, 0, ch, nullptr, false);
-        else  // a velocity chain masks after its last step only: one chain per step
-            for (int64_t k = 0; k < ch; ++k) velocity_steps(c, psi, k, 1, nullptr, true);
+        if (!velocity) {
+            length_steps(c, psi, 0, ch, RedFn(), masked, false, false, src);
+        } else if (!masked) {
+            velocity_steps(c, psi, 0, ch, nullptr, false, RedFn(), src);
+        } else {  // a velocity chain masks after its last step only: one chain per step
+            for (int64_t k = 0; k < ch; ++k) velocity_steps(c, psi, k, 1, nullptr, true, RedFn(), k ? nullptr : src);
+        }
+        src = nullptr;
     }
 }
 
@@ -2482,49 +2500,59 @@ static void adjoint_run(qnd_ctx* c, const void* psi0, const double* F, int64_t n
     const int64_t K = std::max<int64_t>(1, std::min(every, nsteps));
     const int64_t nck = (nsteps + K - 1) / K;
     const bool masked = has_mask(c);
-    DevBuf ck, seg, sub, work, lam, wgrid, wscaled, out, tl, tp;
-    ck.ensure(size_t(nck) * sb);
-    seg.ensure(size_t(K) * sb);
-    sub.ensure(size_t(s) * sb);
-    work.ensure(sb);
-    lam.ensure(sb);
-    if (velocity) {
-        tl.ensure(sb);
-        tp.ensure(sb);
-    }
-    out.ensure((size_t(nsteps) * s * d + 1) * sizeof(double));
-    auto at = [&](DevBuf& b, int64_t k) { return static_cast<void*>(static_cast<char*>(b.p) + size_t(k) * sb); };
-    // the weight: FP64 for J, and dNr w in the state's precision for lambda_T
-    std::vector<double> w(w_host, w_host + c->n), wl(size_t(c->n));
-    for (size_t i = 0; i < wl.size(); ++i) wl[i] = c->dNr * w[i];
-    upload_f64(c, wgrid, w);
-    upload_real(c, wscaled, wl);
+    // one field table per segment (both directions) where it fits the tables of a chunk, else per step
+    const bool seg_tables = 2 * K <= chunk_steps(c);
+    // the states after every sample of a whole segment where they take at most 1 GiB: the segment is then
+    // recomputed once instead of its step starts first and every step's sub-steps from them
+    const bool wide = seg_tables && size_t(K) * s * sb <= (size_t(1) << 30) && !(velocity && masked);
+    // the workspace stays with the context up to 1.5 GiB (allocating it took a tenth of a call at 128^3)
+    size_t bytes = 0;
+    auto take = [&](size_t b) {
+        const size_t o = bytes;
+        bytes += (b + 255) / 256 * 256;
+        return o;
+    };
+    const size_t o_ck = take(size_t(nck) * sb), o_seg = take(wide ? 0 : size_t(K) * sb),
+                 o_sub = take(size_t(wide ? K * s : s) * sb), o_work = take(sb), o_lam = take(sb),
+                 o_tl = take(velocity ? sb : 0), o_tp = take(velocity ? sb : 0), o_w = take(size_t(c->n) * 8),
+                 o_out = take((size_t(nsteps) * s * d + 1) * sizeof(double));
+    DevBuf own;
+    DevBuf& buf = bytes <= (size_t(3) << 29) ? c->adjoint_buf : own;
+    buf.ensure(bytes);
+    auto at = [&](size_t o, int64_t k) { return static_cast<void*>(static_cast<char*>(buf.p) + o + size_t(k) * sb); };
+    // checkpoint q; the first is the caller's state itself
+    auto ck_at = [&](int64_t q) { return q ? static_cast<const void*>(at(o_ck, q)) : psi0; };
+    void* work = at(o_work, 0);
+    void* lam = at(o_lam, 0);
+    if (!c->fp64)  // the weight in the state's precision
+        for (int64_t i = 0; i < c->n; ++i)
+            if (std::isinf(float(c->dNr * w_host[i])) && !std::isinf(c->dNr * w_host[i]))
+                QND_FAIL(QND_EUNSUPPORTED, "a decay factor exceeds the FP32 range: use QND_FP64 for this case");
+    double* wgrid = static_cast<double*>(at(o_w, 0));
+    QND_CK(cudaMemcpyAsync(wgrid, w_host, size_t(c->n) * 8, cudaMemcpyHostToDevice, c->stream));
 
-    // forward, keeping the checkpoints
-    copy_state(c, work.p, psi0);
-    for (int64_t q = 0; q < nck; ++q) {
-        copy_state(c, at(ck, q), work.p);
-        steps_span(c, work.p, F, q * K, std::min(K, nsteps - q * K), masked, velocity);
-    }
-    if (psiT) copy_state(c, psiT, work.p);
-    double* grad_dev = out.as<double>();
+    // forward: every segment from its checkpoint into the next one
+    for (int64_t q = 0; q < nck; ++q)
+        steps_span(c, q + 1 < nck ? at(o_ck, q + 1) : work, ck_at(q), F, q * K, std::min(K, nsteps - q * K), masked,
+                   velocity);
+    double* grad_dev = static_cast<double*>(at(o_out, 0));
     double* J_dev = grad_dev + size_t(nsteps) * s * d;
     RedDesc rj{};
     rj.n = 1;
     rj.kind[0] = RK_ABS2;
     rj.wkind[0] = WK_GRID;
-    rj.wtab[0] = wgrid.as<double>();
+    rj.wtab[0] = wgrid;
     rj.scale[0] = c->dNr;
     rj.out = J_dev;
-    grid_reduce(c, work.p, rj);
-    copy_state(c, lam.p, work.p);
+    grid_reduce(c, work, rj);
     if (c->fp64)
-        launch_point_factors<double>(c->n, lam.as<double2>(), wscaled.as<double>(), nullptr, nullptr, LongArgs{},
-                                     nullptr, nullptr, c->stream);
+        launch_weight_state<double>(c->n, static_cast<double2*>(lam), static_cast<const double2*>(work), wgrid, c->dNr,
+                                    c->stream);
     else
-        launch_point_factors<float>(c->n, lam.as<float2>(), wscaled.as<float>(), nullptr, nullptr, LongArgs{}, nullptr,
-                                    nullptr, c->stream);
+        launch_weight_state<float>(c->n, static_cast<float2*>(lam), static_cast<const float2*>(work), wgrid, c->dNr,
+                                   c->stream);
     c->kernels_launched++;
+    QND_CK(cudaGetLastError());
 
     auto kin = [&](double coef) {
         ChainK k;
@@ -2549,57 +2577,103 @@ static void adjoint_run(qnd_ctx* c, const void* psi0, const double* F, int64_t n
         f.b = i == 0 ? NO_COEF : c->as[2 * i];
         return f;
     };
-    std::vector<double> fe(size_t(2) * s * d);
+    // field tables of steps k0 .. k0+n-1: slots 0 .. n-1 forward, n .. 2n-1 the adjoint's (length: the
+    // laser phases of -E; velocity: the conjugate k-space phases)
+    std::vector<double> fe;
+    auto tables = [&](int64_t k0, int64_t n) {
+        const size_t per = size_t(s) * d;
+        fe.resize(2 * size_t(n) * per);
+        for (size_t q2 = 0; q2 < size_t(n) * per; ++q2) {
+            fe[q2] = F[size_t(k0) * per + q2];
+            fe[size_t(n) * per + q2] = velocity ? fe[q2] : -fe[q2];
+        }
+        upload_field_chunk(c, fe.data(), 2 * n, velocity, velocity ? int(n) : (1 << 30));
+    };
+    // psi' after the parameter-dependent operator i of the step whose tables are in slot lst, from `from`;
+    // joined: from the state after the last such operator of the step before
+    auto substep = [&](int64_t lst, int i, bool joined, const void* from, void* to) {
+        std::vector<ChainK> K;
+        std::vector<ChainMid> M;
+        Factor pre;
+        ChainMid post;
+        if (velocity) {
+            K = kvel(lst, i);
+            pre = vpre(i, RT_VEL);
+            if (joined) {
+                pre.a = c->as[2 * s - 1];
+                pre.b = c->as[0];
+            }
+        } else {
+            post.f.kind = RT_LENGTH;
+            post.f.a = hst(i);
+            post.f.laser_ia = i;
+            post.lst = lst;
+            if (joined && masked) {
+                K = kin(c->as[2 * s - 1]);
+                ChainMid m;
+                m.mask = true;
+                M.push_back(m);
+                K.push_back(kin(cst(i))[0]);
+            } else {
+                K = kin(joined ? c->as[2 * s - 1] + cst(i) : cst(i));
+            }
+        }
+        if (c->dim == 1 && !c->long1d && !chain1d(c) && !M.empty()) {  // 1-D passes carry no mask inside a chain
+            run_chain(c, to, {K[0]}, {}, Factor{}, lst, nullptr, ChainMid{}, false, false, from);
+            apply_step_masks(c, to);
+            run_chain(c, to, {K[1]}, {}, Factor{}, lst, nullptr, post);
+            return;
+        }
+        run_chain(c, to, K, M, pre, lst, nullptr, post, false, false, from);
+    };
     // backward, segment by segment
     for (int64_t q = nck - 1; q >= 0; --q) {
         const int64_t k0 = q * K, kn = std::min(K, nsteps - k0);
-        copy_state(c, work.p, at(ck, q));
-        for (int64_t k = 0; k < kn; ++k) {
-            copy_state(c, at(seg, k), work.p);
-            if (k + 1 < kn) steps_span(c, work.p, F, k0 + k, 1, masked, velocity);
+        if (seg_tables) tables(k0, kn);
+        auto seg_at = [&](int64_t k) { return k ? static_cast<const void*>(at(o_seg, k)) : ck_at(q); };
+        if (wide) {
+            for (int64_t k = 0; k < kn; ++k)
+                for (int i = 0; i < s; ++i) {
+                    const int64_t u = k * s + i;
+                    substep(k, i, k > 0 && i == 0, u ? at(o_sub, u - 1) : ck_at(q), at(o_sub, u));
+                }
+        } else {
+            for (int64_t k = 0; k + 1 < kn; ++k) {
+                if (!seg_tables) steps_span(c, at(o_seg, k + 1), seg_at(k), F, k0 + k, 1, masked, velocity);
+                else if (velocity) velocity_steps(c, at(o_seg, k + 1), k, 1, nullptr, masked, RedFn(), seg_at(k));
+                else length_steps(c, at(o_seg, k + 1), k, 1, RedFn(), masked, false, false, seg_at(k));
+            }
         }
         for (int64_t k = kn - 1; k >= 0; --k) {
             const int64_t kk = k0 + k;
             const double* Fk = F + size_t(kk) * s * d;
-            // field tables of this step: slot 0 forward; slot 1 the adjoint's (length: the laser
-            // phases of -E; velocity: the conjugate k-space phases)
-            for (int q2 = 0; q2 < s * d; ++q2) {
-                fe[q2] = Fk[q2];
-                fe[s * d + q2] = velocity ? Fk[q2] : -Fk[q2];
-            }
-            upload_field_chunk(c, fe.data(), 2, velocity, velocity ? 1 : (1 << 30));
+            if (!seg_tables) tables(kk, 1);
+            const int64_t lf = seg_tables ? k : 0, la = seg_tables ? kn + k : 1;
             // the states just after each parameter-dependent operator
-            copy_state(c, work.p, at(seg, k));
-            for (int i = 0; i < s; ++i) {
-                if (velocity) {
-                    run_chain(c, work.p, kvel(0, i), {}, vpre(i, RT_VEL), 0, nullptr, ChainMid{});
-                } else {
-                    ChainMid post;
-                    post.f.kind = RT_LENGTH;
-                    post.f.a = hst(i);
-                    post.f.laser_ia = i;
-                    post.lst = 0;
-                    run_chain(c, work.p, kin(cst(i)), {}, Factor{}, 0, nullptr, post);
-                }
-                copy_state(c, at(sub, i), work.p);
-            }
+            auto sub_at = [&](int i) { return at(o_sub, wide ? k * s + i : i); };
+            if (!wide)
+                for (int i = 0; i < s; ++i) substep(lf, i, false, i ? sub_at(i - 1) : seg_at(k), sub_at(i));
             // lambda back through the step's last operators: M, then K(a_{2s-1}) or V(a_{2s-1})
-            if (masked) apply_step_masks(c, lam.p);
-            if (velocity) apply_table(c, lam.p, rtab(c, RT_VEL_ADJ, c->as[2 * s - 1], NO_COEF));
-            else run_chain(c, lam.p, kin(-c->as[2 * s - 1]), {}, Factor{}, 0, nullptr, ChainMid{});
+            if (masked) apply_step_masks(c, lam);
+            if (velocity) apply_table(c, lam, rtab(c, RT_VEL_ADJ, c->as[2 * s - 1], NO_COEF));
+            else run_chain(c, lam, kin(-c->as[2 * s - 1]), {}, Factor{}, 0, nullptr, ChainMid{});
             for (int i = s - 1; i >= 0; --i) {
-                RedDesc rg{};
+                AxisImArgs ra{};
+                ra.n = c->n;
+                ra.dim = d;
+                RedDesc& rg = ra.red;
                 rg.n = d;
-                const void* pr = at(sub, i);
-                const void* pl = lam.p;
+                const void* pr = sub_at(i);
+                const void* pl = lam;
                 if (velocity) {
                     // unitary transforms of both states, weights p_j + A_j
-                    copy_state(c, tl.p, lam.p);
-                    copy_state(c, tp.p, at(sub, i));
-                    unitary_fft(c, tl.p, true);
-                    unitary_fft(c, tp.p, true);
-                    pr = tp.p;
-                    pl = tl.p;
+                    void *tl = at(o_tl, 0), *tp = at(o_tp, 0);
+                    copy_state(c, tl, lam);
+                    copy_state(c, tp, sub_at(i));
+                    unitary_fft(c, tl, true);
+                    unitary_fft(c, tp, true);
+                    pr = tp;
+                    pl = tl;
                     for (int j = 0; j < d; ++j) {
                         c->wtab_dev[j].ensure(size_t(c->nr[j]) * 8);
                         launch_axis_table<double>(0, c->p_dev.as<double>() + c->axoff[j], int(c->nr[j]),
@@ -2608,28 +2682,39 @@ static void adjoint_run(qnd_ctx* c, const void* psi0, const double* F, int64_t n
                     }
                 }
                 for (int j = 0; j < d; ++j) {
-                    rg.kind[j] = RK_BILIN_IM;
-                    rg.wkind[j] = WK_AXIS;
-                    rg.waxis[j] = j;
+                    ra.shift[j] = c->shift[j];
+                    ra.nmask[j] = c->nr[j] - 1;
                     rg.wtab[j] = velocity ? c->wtab_dev[j].as<double>() : c->r_dev.as<double>() + c->axoff[j];
                     rg.scale[j] = 2.0 * hst(i);
                 }
                 rg.out = grad_dev + (size_t(kk) * s + i) * d;
-                grid_reduce(c, pr, rg, pl);
+                const int nb = reduce_blocks(c);
+                ensure_red_scratch(c, nb);
+                rg.partials = c->partials.as<double>();
+                rg.counter = c->counter.as<unsigned int>();
+                if (c->fp64)
+                    launch_axis_im_reduce<double>(ra, static_cast<const double2*>(pl), static_cast<const double2*>(pr),
+                                                  c->stream, nb);
+                else
+                    launch_axis_im_reduce<float>(ra, static_cast<const float2*>(pl), static_cast<const float2*>(pr),
+                                                 c->stream, nb);
+                c->kernels_launched++;
+                QND_CK(cudaGetLastError());
                 if (velocity) {
                     ChainMid post;
                     post.f = vpre(i, RT_VEL_ADJ);
-                    run_chain(c, lam.p, kvel(1, i), {}, Factor{}, 0, nullptr, post);
+                    run_chain(c, lam, kvel(la, i), {}, Factor{}, 0, nullptr, post);
                 } else {
                     Factor adj;
                     adj.kind = RT_LENGTH_ADJ;
                     adj.a = hst(i);
                     adj.laser_ia = i;
-                    run_chain(c, lam.p, kin(-cst(i)), {}, adj, 1, nullptr, ChainMid{});
+                    run_chain(c, lam, kin(-cst(i)), {}, adj, la, nullptr, ChainMid{});
                 }
             }
         }
     }
+    if (psiT) copy_state(c, psiT, work);  // last: psiT may be psi0, the first checkpoint
     QND_CK(cudaMemcpyAsync(grad_host, grad_dev, size_t(nsteps) * s * d * sizeof(double), cudaMemcpyDeviceToHost,
                            c->stream));
     double J = 0.0;

@@ -170,6 +170,20 @@ template <typename R> void launch_apply_masks(long long n, cplx_t<R>* psi, int d
 template <typename R> void launch_add_potential(long long n, cplx_t<R>* dst, const cplx_t<R>* src, const double* vtab,
                                                 cudaStream_t st);
 
+// dst = scale w psi (FP64 weights; the product rounded to the state's precision before it multiplies)
+template <typename R> void launch_weight_state(long long n, cplx_t<R>* dst, const cplx_t<R>* psi, const double* w,
+                                               double scale, cudaStream_t st);
+// red.out[j] = red.scale[j] sum_x w_j[x_j] Im(conj(a(x)) b(x)), w_j = red.wtab[j], for every axis j of the grid
+struct AxisImArgs {
+    long long n;
+    int dim;
+    int shift[MAX_DIM];
+    long long nmask[MAX_DIM];
+    RedDesc red;
+};
+template <typename R> void launch_axis_im_reduce(const AxisImArgs& args, const cplx_t<R>* a, const cplx_t<R>* b,
+                                                 cudaStream_t st, int nblocks);
+
 // ---- passes along an axis longer than one pass holds, on a grid of several dimensions
 // (emulate_long_pass in qnd_engine.cu): element-wise work along that axis in natural order.
 // psi *= tr[lm] * tc[lm] * prod_k axc[k][i_k] * prod_k axr[k][i_k] * spec[i_axis] * spec_scale * *scale_dev,

@@ -70,9 +70,9 @@ __host__ __device__ constexpr int pass_kernel_mode(int m, bool reduces, bool end
            : (m == PM_SANDWICH || m == PM_DOUBLE) ? (reduces ? PM_SANDWICH_RED : PM_SANDWICH)
            : m == PM_ROUNDTRIP ? (reduces ? PM_ROUNDTRIP_RED : PM_ROUNDTRIP) : m;
 }
-// |v|^2 w, Re(conj(partner) v) w, or (element-wise grid reductions only) Im(conj(partner) v) w and
-// the count of elements with a non-finite part
-enum : int { RK_ABS2 = 0, RK_BILIN = 1, RK_BILIN_IM = 2, RK_NONFINITE = 3 };
+// |v|^2 w, Re(conj(partner) v) w, or (element-wise grid reductions only) the count of elements with a
+// non-finite part
+enum : int { RK_ABS2 = 0, RK_BILIN = 1, RK_NONFINITE = 2 };
 enum : int { WK_ONE = 0, WK_AXIS = 1, WK_GRID = 2 }; // weight 1, table[idx_axis], line-major table
 
 struct RedDesc {
@@ -95,6 +95,7 @@ struct RedDesc {
 template <typename R> struct PassArgs {
     using V = cplx_t<R>;
     V* psi;
+    const V* src;                // contiguous axes: where the state is read (psi, or another state that stays)
     V* dst;
     const V* partner;
     const V* tw;
@@ -293,11 +294,8 @@ __device__ __forceinline__ void accumulate_red(const RedDesc& rd, double* acc, V
         } else if (rd.kind[k] == RK_BILIN) {
             V p = partner[flat];
             val = double(p.x) * double(v.x) + double(p.y) * double(v.y);
-        } else if (rd.kind[k] == RK_NONFINITE) {
+        } else {  // RK_NONFINITE
             val = (isfinite(double(v.x)) && isfinite(double(v.y))) ? 0.0 : 1.0;
-        } else {
-            V p = partner[flat];
-            val = double(p.x) * double(v.y) - double(p.y) * double(v.x);
         }
         const int wk = rd.wkind[k];
         if (wk == WK_AXIS) {
@@ -661,7 +659,7 @@ __device__ __forceinline__ void pass_group(const PassArgs<R>& a, long long g, un
             for (int u = 0; u < E; ++u) v[u] = active ? line[spad<E>(tid + u * T)] : V{R(0), R(0)};
         }
     } else {
-        const V* __restrict__ src = a.psi;
+        const V* __restrict__ src = a.src;
 #pragma unroll
         for (int u = 0; u < E; ++u) v[u] = active ? src[base + tid + u * T] : V{R(0), R(0)};
         if constexpr (TWS) __syncthreads();  // twiddles visible

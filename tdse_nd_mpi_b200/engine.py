@@ -320,7 +320,7 @@ class Grid:
         F = _f64(F)
         n = F.shape[0]
         F = self._field(F, n)
-        w = _f64(np.broadcast_to(np.asarray(weight, dtype=np.float64), self.shape).copy())
+        w = _f64(np.broadcast_to(np.asarray(weight, dtype=np.float64), self.shape))
         grad = np.zeros((n, self.s, self.dim))
         J = C.c_double()
         check(fn(self.h, C.c_void_p(_ptr_of(psi0)), _dptr(F), int(n), _dptr(w), int(checkpoint), C.byref(J), _dptr(grad),
