@@ -550,6 +550,7 @@ struct PassSpec {
     const void* spec2 = nullptr;
     const void* mid_real = nullptr;
     const void* mid_cplx = nullptr;
+    const void* mid2_cplx = nullptr;  // with reductions between: a factor after them
     const void* mid_ax_cplx[MAX_DIM] = {};
     const void* mid_ax_real[MAX_DIM] = {};
     int red_at_mid = 0;
@@ -620,6 +621,7 @@ template <typename R> static void fill_args(qnd_ctx* c, const PassSpec& ps, Pass
     a.spec2 = static_cast<const V*>(ps.spec2);
     a.mid_real = static_cast<const R*>(ps.mid_real);
     a.mid_cplx = static_cast<const V*>(ps.mid_cplx);
+    a.mid2_cplx = static_cast<const V*>(ps.mid2_cplx);
     for (int k = 0; k < MAX_DIM; ++k) {
         a.mid_ax_cplx[k] = static_cast<const V*>(ps.mid_ax_cplx[k]);
         a.mid_ax_real[k] = static_cast<const R*>(ps.mid_ax_real[k]);
@@ -1277,6 +1279,7 @@ static void emulate_long_pass(qnd_ctx* c, const PassSpec& ps) {
         if (mode == PM_DOUBLE) {
             lax_factors(c, psi, ax, ps.mid_real, ps.mid_cplx, ps.mid_ax_cplx, ps.mid_ax_real, nullptr, 0, 1.0, nullptr);
             if (ps.red_at_mid) reduce(psi);
+            lax_factors(c, psi, ax, nullptr, ps.mid2_cplx, nullptr, nullptr, nullptr, 0, 1.0, nullptr);
             sandwich(psi, ps.spec2);
         }
         lax_factors(c, psi, ax, ps.epi_real, ps.epi_cplx, ps.ax_in_prologue ? nullptr : ps.ax_cplx, ps.ax_real, nullptr, 0,
@@ -1738,9 +1741,8 @@ struct ChainMid {
     int64_t lst = 0;
     bool mask = false;
     const RedDesc* red = nullptr;
-    // chain kernel only (1-D): Gram-Schmidt against the states run_chain1d is given, then a second factor
-    bool gs = false;
-    Factor f2;
+    bool gs = false;  // chain kernel only (1-D): Gram-Schmidt against the states run_chain1d is given
+    Factor f2;        // a second factor after the reductions (or Gram-Schmidt): a full-grid table
     bool empty() const { return f.kind < 0 && f.laser_ia < 0 && !mask && !red && !gs && f2.kind < 0; }
 };
 
@@ -1938,6 +1940,7 @@ static void run_chain(qnd_ctx* c, void* psi, const std::vector<ChainK>& K, const
             set_factor(c, m.f, LONG_ROWS, m.lst, &r.mid_real, &r.mid_cplx, r.mid_ax_cplx);
             if (m.mask) r.mid_ax_real[0] = c->mask_rows.p;
             if (m.red) r.red = *m.red;
+            if (m.f2.kind >= 0) r.mid2_cplx = rtab(c, m.f2.kind, m.f2.a, m.f2.b, LONG_ROWS);
             launch_pass(c, r);
         }
         launch_pass(c, long_pass(c, 0, PM_FFT_INV, psi, 1.0 / double(c->n1)));
@@ -2012,6 +2015,7 @@ static void run_chain(qnd_ctx* c, void* psi, const std::vector<ChainK>& K, const
                     ps.red = *m.red;
                     ps.red_at_mid = 1;
                 }
+                if (m.f2.kind >= 0) ps.mid2_cplx = rtab(c, m.f2.kind, m.f2.a, m.f2.b, ax);
                 ps.spec2 = chain_spec(c, K[i + 1], ax);
                 ps.to_p = to_p && i + 2 == NK;
             }
@@ -2155,22 +2159,27 @@ static void length_steps(qnd_ctx* c, void* psi, int64_t lst0, int64_t n, const R
     run_chain(c, psi, K, M, Factor{}, lst0, nullptr, post, from_p, to_p, src);
 }
 
-// Velocity-gauge steps lst0 .. lst0+n-1 in r-space (integrators.c:201-232); between steps the
-// factors V(a_{2s-1}) V(a_0) merge into one. The step mask and the reductions `fin` apply after the
-// last step only; on the grids of the chain kernel (chain1d), red_fn (in place of fin) and the mask
-// apply after every step.
+// Whether a chain of velocity-gauge steps can carry the step mask and reductions between its steps (1-D
+// passes carry neither inside a chain).
+static bool velocity_chains(const qnd_ctx* c) { return c->dim >= 2 || c->long1d || chain1d(c); }
+
+// Velocity-gauge steps lst0 .. lst0+n-1 in r-space (integrators.c:201-232); between steps the factors
+// V(a_{2s-1}) V(a_0) merge into one, or stand on both sides of the reductions red_fn(k, .) of the state
+// after step k. The step mask applies after every step (velocity_chains; otherwise n is 1). `fin`: the
+// reductions after the last step, in place of red_fn.
 static void velocity_steps(qnd_ctx* c, void* psi, int64_t lst0, int64_t n, const RedDesc* fin, bool masked,
                            const RedFn& red_fn = RedFn(), const void* src = nullptr) {
     if (n <= 0) return;
+    if (n > 1 && (masked || red_fn) && !velocity_chains(c)) QND_FAIL(QND_EINVAL, "internal: a velocity chain with a mask");
     const int s = c->s;
     std::vector<std::vector<RedDesc>> reds;
     reds.reserve(size_t(n));
-    auto reductions = [&](int64_t k) -> const RedDesc* {
+    std::vector<ChainK> K;
+    auto reductions = [&](int64_t k, bool inside) -> const RedDesc* {
         if (!red_fn) return nullptr;
-        reds.push_back(red_fn(k, 0));
+        reds.push_back(red_fn(k, c->long1d && inside ? LONG_ROWS : sandwich_last_axis(c, int64_t(K.size()) - 1)));
         return reds.back().empty() ? nullptr : &reds.back()[0];
     };
-    std::vector<ChainK> K;
     std::vector<ChainMid> M;
     for (int64_t k = 0; k < n; ++k)
         for (int i = 0; i < s; ++i) {
@@ -2179,10 +2188,10 @@ static void velocity_steps(qnd_ctx* c, void* psi, int64_t lst0, int64_t n, const
                 m.f.kind = RT_VEL;
                 m.f.a = i > 0 ? c->as[2 * i - 1] : c->as[2 * s - 1];
                 m.f.b = c->as[2 * i];
-                if (i == 0 && chain1d(c)) {
-                    m.red = reductions(k - 1);
+                if (i == 0) {
+                    m.red = reductions(k - 1, true);
                     m.mask = masked;
-                    if (m.red || m.mask) {  // something between the two factors of the step boundary
+                    if (m.red) {  // of the state between the two factors of the step boundary
                         m.f.b = NO_COEF;
                         m.f2.kind = RT_VEL;
                         m.f2.a = c->as[0];
@@ -2203,7 +2212,7 @@ static void velocity_steps(qnd_ctx* c, void* psi, int64_t lst0, int64_t n, const
     post.f.a = c->as[2 * s - 1];
     post.lst = lst0 + n - 1;
     post.mask = masked;
-    post.red = red_fn ? reductions(n - 1) : fin;
+    post.red = red_fn ? reductions(n - 1, false) : fin;
     run_chain(c, psi, K, M, pre, lst0, nullptr, post, false, false, src);
 }
 
@@ -2348,9 +2357,8 @@ static void run_realtime(qnd_ctx* c, void* psi, const double* field_host, const 
     }
     std::vector<double> zero_alpha(MAX_DIM, 0.0);
     double* rows = c->obs_dev.as<double>();
-    // observables that are r-space reductions of one descriptor: chunk-wide chains (velocity gauge: on
-    // the grids of the chain kernel)
-    const bool chain = (velocity ? chain1d(c) : true) &&
+    // observables that are r-space reductions of one descriptor: chunk-wide chains
+    const bool chain = (!velocity || velocity_chains(c)) &&
                        (nv == 0 || (all_rspace(items) && rspace_red(c, items, rows, 0).size() <= 1));
     for (int64_t c0 = 0; c0 < nsteps; c0 += ch_max) {
         const int64_t ch = std::min(ch_max, nsteps - c0);
@@ -2475,9 +2483,9 @@ static void steps_span(qnd_ctx* c, void* psi, const void* src, const double* F, 
         upload_field_chunk(c, F + size_t(k0 + q) * c->s * c->dim, ch, velocity);
         if (!velocity) {
             length_steps(c, psi, 0, ch, RedFn(), masked, false, false, src);
-        } else if (!masked) {
-            velocity_steps(c, psi, 0, ch, nullptr, false, RedFn(), src);
-        } else {  // a velocity chain masks after its last step only: one chain per step
+        } else if (!masked || velocity_chains(c)) {
+            velocity_steps(c, psi, 0, ch, nullptr, masked, RedFn(), src);
+        } else {  // one chain per step
             for (int64_t k = 0; k < ch; ++k) velocity_steps(c, psi, k, 1, nullptr, true, RedFn(), k ? nullptr : src);
         }
         src = nullptr;

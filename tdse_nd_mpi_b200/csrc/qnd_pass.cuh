@@ -114,6 +114,7 @@ template <typename R> struct PassArgs {
     const V* spec2;              // PM_DOUBLE: the second sandwich's spectral factors
     const R* mid_real;           // PM_DOUBLE: r-space factors between the two sandwiches
     const V* mid_cplx;
+    const V* mid2_cplx;          // reducing passes: a second full-grid factor there, after the reductions
     const V* mid_ax_cplx[MAX_DIM];
     const R* mid_ax_real[MAX_DIM];  // PM_DOUBLE: per-axis real factors between the sandwiches (step mask)
     int red_at_mid;                 // PM_DOUBLE: reduce the state between the sandwiches, not at the end
@@ -590,6 +591,7 @@ __device__ __forceinline__ void pass_group(const PassArgs<R>& a, long long g, un
 #pragma unroll
                 for (int k = 0; k < MAX_RED; ++k)
                     if (k < a.red.n && a.red.wkind[k] == WK_GRID) prefetch_row_l2<L, T>(a.red.wtab[k] + lbase, tid);
+                if (a.mid2_cplx) prefetch_row_l2<L, T>(a.mid2_cplx + lbase, tid);
             }
         }
     }
@@ -692,6 +694,12 @@ __device__ __forceinline__ void pass_group(const PassArgs<R>& a, long long g, un
     // to 256 points 2.74 / 2.66. FP32 passes keep both directions: 2048^2 13.2 / 12.5 ms, and the low parts
     // of their split constants round differently in the conjugate (the sweep of 256^2 to 1024^2 members
     // would gain 3%).
+    auto second_mid = [&] {
+        if (active && a.mid2_cplx) {
+#pragma unroll
+            for (int u = 0; u < E; ++u) v[u] = fmul(v[u], __ldg(a.mid2_cplx + lbase + tid + u * T));
+        }
+    };
     // fwd / inv: whether the transforms run (PassArgs from_p, to_p).
     auto sandwich = [&](bool fwd, bool inv, auto between) {
         if constexpr (ONE_TRANSFORM) {
@@ -726,7 +734,10 @@ __device__ __forceinline__ void pass_group(const PassArgs<R>& a, long long g, un
         if (active)  // a 1-D axis: no other axes
             apply_tables<R, E, T, true>(v, tid, lbase, a.mid_real, a.mid_cplx, a.mid_ax_cplx[0], a.mid_ax_real[0],
                                         false, V{}, false, R(1), key0 ^ 0x2545f491u);
-        if (HAS_RED && a.red.n) reduce();
+        if (HAS_RED && a.red.n) {
+            reduce();
+            second_mid();
+        }
         fft_line_stages<L, E, -1, 0, TWS>(v, tid, line, tw, lsync);
         store_out = true;
     } else if constexpr (MODE == PM_SPECRED) {
@@ -789,7 +800,10 @@ __device__ __forceinline__ void pass_group(const PassArgs<R>& a, long long g, un
                                       use_lf, lf, use_lr, lr,
                                       key0 ^ (place == 0 ? 0x51ed270bu : (place == 1 ? 0x2545f491u : 0x68e31da4u)));
             }
-            if (HAS_RED && a.red.n && place == (a.red_at_mid ? 1 : 2)) reduce();
+            if (HAS_RED && a.red.n && place == (a.red_at_mid ? 1 : 2)) {
+                reduce();
+                if (place == 1) second_mid();
+            }
             if (place == 2) break;
             const bool fwd = !ENDS || half > 0 || !a.from_p, inv = !ENDS || half + 1 < a.sandwiches || !a.to_p;
             sandwich(fwd, inv, [&] {
