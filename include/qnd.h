@@ -178,7 +178,8 @@ int qnd_run_length_batch(int count, qnd_ctx *const *ctxs, void *const *psi_r_dev
  *      QND_NO_GRAPH set), then one cooperative launch per segment of 512 steps runs all of them: the
  *      CTAs claim line groups in round order (pass r of every member, then pass r + 1) and wait, with
  *      a bounded wait, only for the member's own previous pass, so members advance independently and
- *      small grids fill the GPU together. Members must share one precision; every axis length is 128
+ *      small grids fill the GPU together. 1-D members run their chain kernels beside it, one SM each,
+ *      as qnd_run_length_dev does. Members must share one precision; every axis length is 128
  *      to 1024 (QND_EUNSUPPORTED otherwise, or for observables beyond one fused reduction: use
  *      qnd_run_length_batch). A wait that runs out makes the call return QND_ECUDA. Synchronises. */
 int qnd_run_length_sweep(int count, qnd_ctx *const *ctxs, void *const *psi_r_dev, const double *const *E_dev,

@@ -1775,7 +1775,7 @@ static int chain_final_axis(const qnd_ctx* c, int NK) { return sandwich_last_axi
 // points. A pass of such a grid is one CTA on one SM, so a launch per pair of sandwiches left the GPU
 // waiting on launches and on the state's round trip: a BM4 step took 77 us at 4096 points (with
 // Gram-Schmidt) and 34 us at 512 (with observables) by passes, and takes 37 and 12.7 us by this kernel. Shorter lines have fewer than a warp of
-// 4-point threads and keep the passes, as do the recorded passes of the persistent sweep kernel.
+// 4-point threads and keep the passes.
 static bool chain1d(const qnd_ctx* c) { return c->tw_chain.p && !c->recorder; }
 
 struct ChainGs {
@@ -3825,7 +3825,9 @@ int qnd_run_length_batch(int count, qnd_ctx* const* ctxs, void* const* psi_r_dev
 // qnd_run_length_sweep: every member's passes recorded (the chains qnd_run_length_dev would launch,
 // chunk by chunk, with the same arguments), then run by the persistent sweep kernel (qnd_sweep.cu) in
 // one launch per segment of SWEEP_SEGMENT steps. Segments keep the recorded arguments and the field
-// tables of all their chunks in device memory at once.
+// tables of all their chunks in device memory at once. A 1-D member runs no passes when alone: its chain
+// kernels go out on its own stream, one SM each, beside the sweep kernel, whose grid leaves them that
+// many SMs (at most half of the GPU's).
 static const int64_t SWEEP_SEGMENT = 512;
 
 int qnd_run_length_sweep(int count, qnd_ctx* const* ctxs, void* const* psi_r_dev, const double* const* E_dev,
@@ -3870,6 +3872,8 @@ int qnd_run_length_sweep(int count, qnd_ctx* const* ctxs, void* const* psi_r_dev
             QND_FAIL(QND_EUNSUPPORTED, "qnd_run_length_sweep: observables beyond one fused reduction descriptor");
     }
     qnd_ctx* home = ctxs[0];
+    for (int i = count - 1; i >= 0; --i)
+        if (!chain1d(ctxs[i])) home = ctxs[i];
     const size_t argsz = (size_t(home->fp64 ? sizeof(PassArgs<double>) : sizeof(PassArgs<float>)) + 127) / 128 * 128;
     struct Ev {
         std::vector<cudaEvent_t> e;
@@ -3883,13 +3887,17 @@ int qnd_run_length_sweep(int count, qnd_ctx* const* ctxs, void* const* psi_r_dev
     int failed = 0;
     for (int64_t s0 = 0; s0 < nsteps && !failed; s0 += SWEEP_SEGMENT) {
         const int64_t seg = std::min(SWEEP_SEGMENT, nsteps - s0);
-        // record every member's chains for this segment (their field tables built on their streams)
+        // record every member's chains for this segment (their field tables built on their streams), or
+        // launch them (1-D members)
         std::vector<std::vector<RecordedPass>> rec(static_cast<size_t>(count));
+        int ndirect = 0;
         for (int i = 0; i < count; ++i) {
             SweepMember& m = ms[i];
             qnd_ctx* c = m.c;
             const int64_t chunk = chunk_steps(c);
             const size_t per_step = size_t(c->s) * c->axtot * c->elem();
+            const bool direct = chain1d(c);
+            ndirect += direct;
             c->sweep_field.ensure(size_t(seg) * per_step);
             for (int64_t c0 = 0; c0 < seg; c0 += chunk) {
                 const int64_t ch = std::min(chunk, seg - c0);
@@ -3901,7 +3909,7 @@ int qnd_run_length_sweep(int count, qnd_ctx* const* ctxs, void* const* psi_r_dev
                     SweepMember* mp = &m;
                     rf = [mp, rows](int64_t k, int ax) { return rspace_red(mp->c, mp->items, rows + size_t(k) * mp->nv, ax); };
                 }
-                c->recorder = &rec[i];
+                if (!direct) c->recorder = &rec[i];
                 c->field_view = tabs;
                 try {
                     length_steps(c, psi_r_dev[i], 0, ch, rf, m.masked);
@@ -3961,10 +3969,19 @@ int qnd_run_length_sweep(int count, qnd_ctx* const* ctxs, void* const* psi_r_dev
         char* dbuf = static_cast<char*>(home->sweep_buf.p);
         for (size_t q = 0; q < slots.size(); ++q) slots[q].args = dbuf + blob_off[q];
         // every member's earlier work (state, tables) before the sweep's stream reads it
-        for (int i = 0; i < count; ++i) {
-            QND_CK(cudaEventRecord(ev.e[i], ms[i].c->stream));
-            QND_CK(cudaStreamWaitEvent(home->stream, ev.e[i], 0));
+        auto join = [&](bool direct) {
+            for (int i = 0; i < count; ++i) {
+                if (rec[i].empty() != direct) continue;
+                QND_CK(cudaEventRecord(ev.e[i], ms[i].c->stream));
+                QND_CK(cudaStreamWaitEvent(home->stream, ev.e[i], 0));
+            }
+        };
+        if (slots.empty()) {
+            join(true);
+            QND_CK(cudaStreamSynchronize(home->stream));
+            continue;
         }
+        join(false);
         QND_CK(cudaMemcpyAsync(dbuf, blob.data(), nb, cudaMemcpyHostToDevice, home->stream));
         QND_CK(cudaMemcpyAsync(dbuf + o_slots, slots.data(), slots.size() * sizeof(SweepSlot), cudaMemcpyHostToDevice,
                                home->stream));
@@ -3982,8 +3999,9 @@ int qnd_run_length_sweep(int count, qnd_ctx* const* ctxs, void* const* psi_r_dev
         sa.abort_flag = reinterpret_cast<int*>(dbuf + o_ctl + o_next + 16);
         sa.wait_tries = 1 << 22;  // ~1 s of polling per item before the launch gives up
         int grid = 0;
-        const cudaError_t le = home->fp64 ? launch_sweep<double>(sa, home->stream, home->num_sms, &grid)
-                                          : launch_sweep<float>(sa, home->stream, home->num_sms, &grid);
+        const int sms = home->num_sms - std::min(ndirect, home->num_sms / 2);
+        const cudaError_t le = home->fp64 ? launch_sweep<double>(sa, home->stream, sms, &grid)
+                                          : launch_sweep<float>(sa, home->stream, sms, &grid);
         if (le != cudaSuccess) {
             cudaGetLastError();
             QND_FAIL(QND_ECUDA, "qnd_run_length_sweep: launch of the sweep kernel: %s", cudaGetErrorString(le));
@@ -3991,6 +4009,7 @@ int qnd_run_length_sweep(int count, qnd_ctx* const* ctxs, void* const* psi_r_dev
         // the members' later work after the sweep; the blob and tables are reused by the next segment
         QND_CK(cudaEventRecord(ev.e[count], home->stream));
         for (int i = 0; i < count; ++i) QND_CK(cudaStreamWaitEvent(ms[i].c->stream, ev.e[count], 0));
+        join(true);
         QND_CK(cudaMemcpyAsync(&failed, sa.abort_flag, sizeof(int), cudaMemcpyDeviceToHost, home->stream));
         QND_CK(cudaStreamSynchronize(home->stream));
     }

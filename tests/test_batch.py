@@ -177,6 +177,31 @@ def test_persistent_sweep_matches_members_alone(qnd_lib, precision, monkeypatch)
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("shapes", [((128,), (1024,)), ((1024,), (256, 128), (128,))])
+def test_persistent_sweep_holds_1d_members(qnd_lib, precision, shapes, monkeypatch):
+    """1-D members of the shortest and longest lines the sweep takes, alone and beside a 2-D member, 520
+    steps (more than one segment): rows and final states equal each member's own run, bit for bit."""
+    import dataclasses
+
+    from tdse_nd_mpi_b200.batch import run_members
+
+    def member(shape, seed):
+        m = _member(shape, seed)
+        rng = np.random.default_rng(300 + seed)
+        return dataclasses.replace(m, field=rng.standard_normal((520, 6, len(shape))) * 0.05, precision=precision)
+
+    members = [member(s, 51 + k) for k, s in enumerate(shapes)]
+    together = run_members(members, one_graph="persistent")
+    monkeypatch.setenv("QND_NO_GRAPH", "1")
+    monkeypatch.setenv("QND_SHAPE", "0")
+    alone = run_members(members, one_graph=False)
+    for a, b in zip(together, alone):
+        np.testing.assert_array_equal(a["obs"], b["obs"])
+        np.testing.assert_array_equal(a["psi"], b["psi"])
+
+
+@pytest.mark.gpu
 def test_persistent_sweep_refuses_what_it_does_not_hold(qnd_lib):
     """Axis lengths outside 128..1024 and mixed precisions give QND_EUNSUPPORTED (no launch)."""
     from tdse_nd_mpi_b200 import QndError
