@@ -192,14 +192,15 @@ int qnd_run_length_sweep(int count, qnd_ctx *const *ctxs, void *const *psi_r_dev
  *      |r| > R: the norm absorbed there), and writes dJ/dE[k][ia][j] for every sample into
  *      grad_host [nsteps][s][dim], by running the adjoint state backward through the steps.
  *      The forward states are kept every `checkpoint` steps and recomputed in between: the device
- *      holds at most ceil(nsteps/checkpoint) + checkpoint + s + 2 states, or, where that takes at most
- *      1 GiB, s * checkpoint states in the place of checkpoint + s (a workspace of up to 1.5 GiB stays
- *      with the context). J_out and psiT_dev (psi(T)) may be
- *      NULL. Synchronises. */
+ *      holds at most ceil(nsteps/checkpoint) + checkpoint + s + 1 states and the weight (8 bytes a
+ *      point), or, where that takes at most 1 GiB and the memory is there, s * checkpoint states in the
+ *      place of checkpoint + s. One workspace of up to 1.5 GiB per device is kept for later calls, until
+ *      a context of that device is destroyed or another allocation of this library needs it. J_out and
+ *      psiT_dev (psi(T)) may be NULL. Synchronises. */
 int qnd_adjoint_length(qnd_ctx *ctx, const void *psi0_dev, const double *E_host, int64_t nsteps, const double *w_host,
                        int64_t checkpoint, double *J_out, double *grad_host, void *psiT_dev);
 /* The same for a velocity-gauge run (qnd_step_velocity's steps, the step mask after each): dJ/dA for
- * every vector-potential sample A_host [nsteps][s][dim]. */
+ * every vector-potential sample A_host [nsteps][s][dim]. Two states more on the device. */
 int qnd_adjoint_velocity(qnd_ctx *ctx, const void *psi0_dev, const double *A_host, int64_t nsteps,
                          const double *w_host, int64_t checkpoint, double *J_out, double *grad_host, void *psiT_dev);
 

@@ -62,6 +62,27 @@ static std::string fmt(const char* f, ...) {
         if (e_ != cudaSuccess) QND_FAIL(QND_ECUDA, "%s: %s", #x, cudaGetErrorString(e_));           \
     } while (0)
 
+static bool release_workspace(int device);
+
+// cudaMalloc on the current device. Where it fails, the workspace kept for later adjoint calls is given
+// back and the request made once more.
+static void* device_alloc(size_t b) {
+    // fault injection for the tests: QND_FAIL_ALLOC_ABOVE=<bytes> makes every larger request fail here, on
+    // the host, as an out-of-memory would
+    const char* lim = std::getenv("QND_FAIL_ALLOC_ABOVE");
+    const bool refused = lim && b > size_t(std::strtoull(lim, nullptr, 10));
+    void* p = nullptr;
+    int device = 0;
+    for (;;) {
+        const cudaError_t e = refused ? cudaErrorMemoryAllocation : cudaMalloc(&p, b ? b : 16);
+        if (e == cudaSuccess) return p;
+        cudaGetLastError();
+        if (cudaGetDevice(&device) == cudaSuccess && release_workspace(device)) continue;
+        if (refused) QND_FAIL(QND_ENOMEM, "cudaMalloc(%zu bytes): refused by QND_FAIL_ALLOC_ABOVE=%s", b, lim);
+        QND_FAIL(QND_ENOMEM, "cudaMalloc(%zu bytes): %s", b, cudaGetErrorString(e));
+    }
+}
+
 struct DevBuf {
     void* p = nullptr;
     size_t bytes = 0;
@@ -81,20 +102,38 @@ struct DevBuf {
         if (p) cudaFree(p);
         p = nullptr;
         bytes = 0;
-        // fault injection for the tests: QND_FAIL_ALLOC_ABOVE=<bytes> makes every larger request fail
-        // here, on the host, as an out-of-memory would
-        if (const char* lim = std::getenv("QND_FAIL_ALLOC_ABOVE"))
-            if (b > size_t(std::strtoull(lim, nullptr, 10)))
-                QND_FAIL(QND_ENOMEM, "cudaMalloc(%zu bytes): refused by QND_FAIL_ALLOC_ABOVE=%s", b, lim);
-        cudaError_t e = cudaMalloc(&p, b ? b : 16);
-        if (e != cudaSuccess) {
-            cudaGetLastError();
-            QND_FAIL(QND_ENOMEM, "cudaMalloc(%zu bytes): %s", b, cudaGetErrorString(e));
-        }
+        p = device_alloc(b);
         bytes = b;
     }
     template <class T> T* as() const { return static_cast<T*>(p); }
 };
+
+// The workspace of adjoint calls. Allocating and freeing it took a tenth of a call at 128^3, so one of up to
+// 1.5 GiB per device is kept after a call that ended with its stream idle. It is held by at most one call
+// at a time, and given back when any context of the device is closed or any allocation here fails.
+static std::mutex g_workspace_lock;
+static std::map<int, std::unique_ptr<DevBuf>>& kept_workspaces() {
+    static auto* m = new std::map<int, std::unique_ptr<DevBuf>>;  // never destroyed: CUDA is gone at exit
+    return *m;
+}
+constexpr size_t KEEP_WORKSPACE = size_t(3) << 29;
+
+static std::unique_ptr<DevBuf> take_workspace(int device) {
+    std::lock_guard<std::mutex> lk(g_workspace_lock);
+    auto w = std::move(kept_workspaces()[device]);
+    return w ? std::move(w) : std::make_unique<DevBuf>();
+}
+static void keep_workspace(int device, std::unique_ptr<DevBuf> w) {
+    if (w->bytes > KEEP_WORKSPACE) return;
+    std::lock_guard<std::mutex> lk(g_workspace_lock);
+    auto& slot = kept_workspaces()[device];
+    if (!slot || slot->bytes < w->bytes) std::swap(slot, w);
+}
+static bool release_workspace(int device) {
+    std::lock_guard<std::mutex> lk(g_workspace_lock);
+    auto w = std::move(kept_workspaces()[device]);
+    return w && w->p;
+}
 
 static PassKernelInfo lookup_pass(bool fp64, int L, bool strided, int mode, int var = 0, bool tma = false) {
 #define QND_CASE(LL)                                                                                              \
@@ -196,7 +235,6 @@ struct qnd_ctx {
     DevBuf tune_buf;                            // scratch state of the staging autotuner
     DevBuf shape_buf;                           // scratch state of the shape autotuner (its own: the
                                                 // staging tuner frees tune_buf inside its launches)
-    DevBuf adjoint_buf;                         // workspace of the adjoint calls (adjoint_run)
     DevBuf finite_slot;                         // QND_CHECK_FINITE: the non-finite count
     std::map<std::tuple<const void*, int, int>, CUtensorMap> tmaps;  // strided-pass TMA views of states
 
@@ -2440,8 +2478,9 @@ static void run_realtime(qnd_ctx* c, void* psi, const double* field_host, const 
 //   dJ/dA[k][i][j] = 2 h_i sum_k (p_j + A[k][i][j]) Im(conj(lambda~') psi~')   (just after P_i).
 // Adjoints: V(a) -> RT_VEL_ADJ, P_i -> the sandwich with the conjugate phase tables.
 //
-// The forward states are kept every `every` steps; a segment's step-start states are recomputed
-// from its checkpoint, and a step's sub-step states from its start.
+// The forward states are kept every `every` steps (the first is the caller's). Going back, a segment is
+// recomputed from its checkpoint: every state after a field sample at once (adjoint_run's `wide`), or its
+// step-start states first and then each step's sub-step states from them.
 
 // psi <- M psi for the step masks set on the axes.
 static void apply_step_masks(qnd_ctx* c, void* psi) {
@@ -2501,8 +2540,9 @@ struct SweepMember {
     double* stage = nullptr;
 };
 
-static void adjoint_run(qnd_ctx* c, const void* psi0, const double* F, int64_t nsteps, const double* w_host,
-                        int64_t every, double* J_out, double* grad_host, void* psiT, bool velocity) {
+// wide: whether a segment's sub-step states may all be held at once; on return whether they were.
+static void adjoint_attempt(qnd_ctx* c, const void* psi0, const double* F, int64_t nsteps, const double* w_host,
+                            int64_t every, double* J_out, double* grad_host, void* psiT, bool velocity, bool& wide) {
     const int s = c->s, d = c->dim;
     const size_t sb = size_t(c->n) * c->elem();
     const int64_t K = std::max<int64_t>(1, std::min(every, nsteps));
@@ -2512,24 +2552,23 @@ static void adjoint_run(qnd_ctx* c, const void* psi0, const double* F, int64_t n
     const bool seg_tables = 2 * K <= chunk_steps(c);
     // the states after every sample of a whole segment where they take at most 1 GiB: the segment is then
     // recomputed once instead of its step starts first and every step's sub-steps from them
-    const bool wide = seg_tables && size_t(K) * s * sb <= (size_t(1) << 30) && !(velocity && masked);
-    // the workspace stays with the context up to 1.5 GiB (allocating it took a tenth of a call at 128^3)
+    wide = wide && seg_tables && size_t(K) * s * sb <= (size_t(1) << 30) && !(velocity && masked);
     size_t bytes = 0;
     auto take = [&](size_t b) {
         const size_t o = bytes;
         bytes += (b + 255) / 256 * 256;
         return o;
     };
-    const size_t o_ck = take(size_t(nck) * sb), o_seg = take(wide ? 0 : size_t(K) * sb),
+    const size_t o_ck = take(size_t(nck - 1) * sb), o_seg = take(wide ? 0 : size_t(K) * sb),
                  o_sub = take(size_t(wide ? K * s : s) * sb), o_work = take(sb), o_lam = take(sb),
                  o_tl = take(velocity ? sb : 0), o_tp = take(velocity ? sb : 0), o_w = take(size_t(c->n) * 8),
                  o_out = take((size_t(nsteps) * s * d + 1) * sizeof(double));
-    DevBuf own;
-    DevBuf& buf = bytes <= (size_t(3) << 29) ? c->adjoint_buf : own;
-    buf.ensure(bytes);
-    auto at = [&](size_t o, int64_t k) { return static_cast<void*>(static_cast<char*>(buf.p) + o + size_t(k) * sb); };
+    // ensure() gives a smaller one back before it allocates
+    auto buf = take_workspace(c->device);
+    buf->ensure(bytes);
+    auto at = [&](size_t o, int64_t k) { return static_cast<void*>(static_cast<char*>(buf->p) + o + size_t(k) * sb); };
     // checkpoint q; the first is the caller's state itself
-    auto ck_at = [&](int64_t q) { return q ? static_cast<const void*>(at(o_ck, q)) : psi0; };
+    auto ck_at = [&](int64_t q) { return q ? static_cast<const void*>(at(o_ck, q - 1)) : psi0; };
     void* work = at(o_work, 0);
     void* lam = at(o_lam, 0);
     if (!c->fp64)  // the weight in the state's precision
@@ -2541,7 +2580,7 @@ static void adjoint_run(qnd_ctx* c, const void* psi0, const double* F, int64_t n
 
     // forward: every segment from its checkpoint into the next one
     for (int64_t q = 0; q < nck; ++q)
-        steps_span(c, q + 1 < nck ? at(o_ck, q + 1) : work, ck_at(q), F, q * K, std::min(K, nsteps - q * K), masked,
+        steps_span(c, q + 1 < nck ? at(o_ck, q) : work, ck_at(q), F, q * K, std::min(K, nsteps - q * K), masked,
                    velocity);
     double* grad_dev = static_cast<double*>(at(o_out, 0));
     double* J_dev = grad_dev + size_t(nsteps) * s * d;
@@ -2728,8 +2767,23 @@ static void adjoint_run(qnd_ctx* c, const void* psi0, const double* F, int64_t n
     double J = 0.0;
     QND_CK(cudaMemcpyAsync(&J, J_dev, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     QND_CK(cudaStreamSynchronize(c->stream));
+    keep_workspace(c->device, std::move(buf));
     check_device_error(c);
     if (J_out) *J_out = J;
+}
+
+static void adjoint_run(qnd_ctx* c, const void* psi0, const double* F, int64_t nsteps, const double* w_host,
+                        int64_t every, double* J_out, double* grad_host, void* psiT, bool velocity) {
+    bool wide = true;
+    try {
+        adjoint_attempt(c, psi0, F, nsteps, w_host, every, J_out, grad_host, psiT, velocity, wide);
+    } catch (const Error& e) {
+        // no memory for the wide layout's states or tables (every allocation precedes the writes to the
+        // caller's results): once more with a step's sub-step states at a time
+        if (e.code != QND_ENOMEM || !wide) throw;
+        wide = false;
+        adjoint_attempt(c, psi0, F, nsteps, w_host, every, J_out, grad_host, psiT, velocity, wide);
+    }
 }
 
 // ---------------------------------------------------------------- Gram-Schmidt --
@@ -3048,6 +3102,7 @@ int qnd_ctx_destroy(qnd_ctx* ctx) {
     for (auto e : ctx->event_pool) cudaEventDestroy(e);
     for (auto& kv : ctx->graphs) cudaGraphExecDestroy(kv.second.exec);
     if (ctx->own_stream && ctx->stream) cudaStreamDestroy(ctx->stream);
+    release_workspace(ctx->device);
     delete ctx;
     QND_API_END
 }
@@ -3206,13 +3261,8 @@ int qnd_state_alloc(qnd_ctx* ctx, int64_t nstates, void** psi_dev) {
     QND_NEED(psi_dev);
     if (nstates < 1) QND_FAIL(QND_EINVAL, "nstates must be >= 1");
     set_device(ctx);
-    void* p = nullptr;
     const size_t bytes = size_t(nstates) * size_t(ctx->n) * ctx->elem();
-    cudaError_t e = cudaMalloc(&p, bytes);
-    if (e != cudaSuccess) {
-        cudaGetLastError();
-        QND_FAIL(QND_ENOMEM, "cudaMalloc(%zu bytes): %s", bytes, cudaGetErrorString(e));
-    }
+    void* p = device_alloc(bytes);
     QND_CK(cudaMemsetAsync(p, 0, bytes, ctx->stream));
     *psi_dev = p;
     QND_API_END

@@ -44,3 +44,73 @@ def test_paths_agree(qnd_lib, shape, steps, checkpoints, integ, velocity, masked
     # the same operators in another grouping: rounding of some hundred transforms
     assert abs(Ja - Jb) <= 1e-11 * abs(Jb)
     assert np.linalg.norm(a - b) <= 1e-10 * np.linalg.norm(b)
+
+
+def _small(n, integ, checkpoint):
+    from tdse_nd_mpi_b200 import Grid
+
+    g = Grid(3, (n,) * 3, (0.3,) * 3, integ, 0.05)
+    r2 = sum(np.reshape(g.axis_r(j) ** 2, [-1 if k == j else 1 for k in range(3)]) for j in range(3))
+    g.set_potential(-1.0 / np.sqrt(r2 + 0.5))
+    st = g.state(np.exp(-0.5 * r2) + 0j)
+    E = np.random.default_rng(9).standard_normal((checkpoint, g.s, 3)) * 0.05
+    w = (r2 > 4.0).astype(np.float64)
+    return g, st, lambda: g.adjoint_length(st, E, w, checkpoint)
+
+
+def test_no_memory_for_the_wide_layout(qnd_lib, monkeypatch):
+    """A segment of 8 BM4 steps at 32^3: 50 states (26 MB) at once, 16 states (8.7 MB) step by step. Where
+    only the second fits the call still runs, with the same gradient to rounding."""
+    g, st, run = _small(32, "BM4", 8)
+    Ja, a = run()
+    g.close()
+    g, st, run = _small(32, "BM4", 8)
+    monkeypatch.setenv("QND_FAIL_ALLOC_ABOVE", str(16 << 20))
+    Jb, b = run()
+    monkeypatch.delenv("QND_FAIL_ALLOC_ABOVE")
+    assert abs(Ja - Jb) <= 1e-11 * abs(Jb)
+    assert np.linalg.norm(a - b) <= 1e-10 * np.linalg.norm(b)
+    g.close()
+
+
+def test_kept_workspace_is_bounded_and_given_back(qnd_lib, monkeypatch):
+    """Contexts that have run an adjoint keep one workspace between them (74 MB here), which a failing
+    allocation gives back."""
+    import torch
+
+    from tdse_nd_mpi_b200 import QndError
+
+    sets = [_small(64, "Verlet", 16) for _ in range(3)]
+    want = [run() for _, _, run in sets][0]
+    monkeypatch.setenv("QND_FAIL_ALLOC_ABOVE", str(1 << 20))
+    freed = []
+    for _ in range(2):
+        before = torch.cuda.mem_get_info()[0]
+        with pytest.raises(QndError) as ei:
+            sets[0][0].state()
+        assert ei.value.code == 3
+        freed.append(torch.cuda.mem_get_info()[0] - before)
+    monkeypatch.delenv("QND_FAIL_ALLOC_ABOVE")
+    assert 72 << 20 <= freed[0] <= 84 << 20 and freed[1] == 0
+    J, grad = sets[1][2]()
+    assert J == want[0] and np.array_equal(grad, want[1])
+    for g, *_ in sets:
+        g.close()
+
+
+def test_calls_on_several_threads(qnd_lib):
+    """Calls that run at the same time on different contexts do not share the kept workspace."""
+    import threading
+
+    sets = [_small(32, "BM4", 4) for _ in range(4)]
+    want = [run() for _, _, run in sets]
+    got = [None] * 4
+    threads = [threading.Thread(target=lambda k: got.__setitem__(k, sets[k][2]()), args=(k,)) for k in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join(timeout=300)
+    for (Ja, a), (Jb, b) in zip(want, got):
+        assert Ja == Jb and np.array_equal(a, b)
+    for g, *_ in sets:
+        g.close()
