@@ -510,6 +510,10 @@ static const void* rtab(qnd_ctx* c, int kind, double a, double b, int ax) {
     auto it = c->rtab_cache.find(key);
     if (it != c->rtab_cache.end()) return it->second->p;
     if (c->vpot.empty()) QND_FAIL(QND_EINVAL, "no potential set: call qnd_set_potential_named or qnd_set_potential");
+    // fault injection for the tests: QND_FAIL_TABLES_ABOVE=<count> refuses a context more tables than that
+    if (const char* lim = std::getenv("QND_FAIL_TABLES_ABOVE"))
+        if (c->rtab_cache.size() >= size_t(std::strtoull(lim, nullptr, 10)))
+            QND_FAIL(QND_ENOMEM, "full-grid table %zu: refused by QND_FAIL_TABLES_ABOVE=%s", c->rtab_cache.size() + 1, lim);
     const size_t n = size_t(c->n);
     auto buf = std::make_unique<DevBuf>();
     if (kind == RT_IMAG) {
@@ -2201,6 +2205,36 @@ static void length_steps(qnd_ctx* c, void* psi, int64_t lst0, int64_t n, const R
 // passes carry neither inside a chain).
 static bool velocity_chains(const qnd_ctx* c) { return c->dim >= 2 || c->long1d || chain1d(c); }
 
+// Whether n velocity-gauge steps run as one chain with the step mask or nothing between them: the merged
+// factor of a step boundary is a full-grid table that single steps do not need. Where there is no memory
+// for it (or, in FP32, the product leaves the range), the steps run one chain each. Reductions at the
+// boundary keep its two factors apart, which are the tables of a step's two ends.
+static bool velocity_joins(qnd_ctx* c, int64_t n) {
+    if (!velocity_chains(c)) return false;
+    const int s = c->s;
+    std::vector<std::tuple<int, double, double, uint64_t>> added;
+    auto table = [&](double a, double b, int ax) {
+        const size_t held = c->rtab_cache.size();
+        rtab(c, RT_VEL, a, b, ax);
+        if (c->rtab_cache.size() > held) added.emplace_back(RT_VEL * 8 + ax, a, b, c->table_epoch);
+    };
+    // a single step's tables first
+    const int rows = c->long1d ? LONG_ROWS : -1;
+    table(c->as[0], NO_COEF, c->dim - 1);
+    table(c->as[2 * s - 1], NO_COEF, chain_final_axis(c, s));
+    for (int i = 1; i < s; ++i) table(c->as[2 * i - 1], c->as[2 * i], rows < 0 ? sandwich_last_axis(c, i - 1) : rows);
+    added.clear();
+    try {
+        for (int64_t k = 1; k < n && k <= 2; ++k)  // boundaries alternate between two passes where s is odd
+            table(c->as[2 * s - 1], c->as[0], rows < 0 ? sandwich_last_axis(c, s * k - 1) : rows);
+    } catch (const Error& e) {
+        if (e.code != QND_ENOMEM && e.code != QND_EUNSUPPORTED) throw;
+        for (const auto& key : added) c->rtab_cache.erase(key);
+        return false;
+    }
+    return true;
+}
+
 // Velocity-gauge steps lst0 .. lst0+n-1 in r-space (integrators.c:201-232); between steps the factors
 // V(a_{2s-1}) V(a_0) merge into one, or stand on both sides of the reductions red_fn(k, .) of the state
 // after step k. The step mask applies after every step (velocity_chains; otherwise n is 1). `fin`: the
@@ -2396,8 +2430,8 @@ static void run_realtime(qnd_ctx* c, void* psi, const double* field_host, const 
     std::vector<double> zero_alpha(MAX_DIM, 0.0);
     double* rows = c->obs_dev.as<double>();
     // observables that are r-space reductions of one descriptor: chunk-wide chains
-    const bool chain = (!velocity || velocity_chains(c)) &&
-                       (nv == 0 || (all_rspace(items) && rspace_red(c, items, rows, 0).size() <= 1));
+    const bool chain = (nv == 0 || (all_rspace(items) && rspace_red(c, items, rows, 0).size() <= 1)) &&
+                       (!velocity || (nv ? velocity_chains(c) : velocity_joins(c, nsteps)));
     for (int64_t c0 = 0; c0 < nsteps; c0 += ch_max) {
         const int64_t ch = std::min(ch_max, nsteps - c0);
         if (nv > 0 && c0 == 0) {
@@ -2517,12 +2551,13 @@ static void apply_table(qnd_ctx* c, void* psi, const void* table) {
 static void steps_span(qnd_ctx* c, void* psi, const void* src, const double* F, int64_t k0, int64_t n, bool masked,
                        bool velocity) {
     const int64_t chunk = chunk_steps(c);
+    const bool joined = !velocity || !masked || velocity_joins(c, n);
     for (int64_t q = 0; q < n; q += chunk) {
         const int64_t ch = std::min(chunk, n - q);
         upload_field_chunk(c, F + size_t(k0 + q) * c->s * c->dim, ch, velocity);
         if (!velocity) {
             length_steps(c, psi, 0, ch, RedFn(), masked, false, false, src);
-        } else if (!masked || velocity_chains(c)) {
+        } else if (joined) {
             velocity_steps(c, psi, 0, ch, nullptr, masked, RedFn(), src);
         } else {  // one chain per step
             for (int64_t k = 0; k < ch; ++k) velocity_steps(c, psi, k, 1, nullptr, true, RedFn(), k ? nullptr : src);

@@ -42,3 +42,42 @@ def test_velocity_run_vs_oracle(qnd_lib, shape, integ, steps, masked):
     g.run_velocity(st2, A, alpha, [])
     assert np.linalg.norm(st2.download() - b) <= 1e-12 * grow * np.linalg.norm(b)
     g.close()
+
+
+@pytest.mark.parametrize("integ", ["Verlet", "RKN4"])
+@pytest.mark.parametrize("shape", [(32, 64), (16384,)])
+@pytest.mark.parametrize("masked", [False, True])
+def test_no_memory_for_the_boundary_factor(qnd_lib, integ, shape, masked, monkeypatch):
+    """Where a context holds only the tables that a single step needs, a run of several steps still goes
+    through (step by step), with the same state to rounding."""
+    from tdse_nd_mpi_b200 import QndError
+
+    def run(steps):
+        from tdse_nd_mpi_b200 import Grid
+
+        dim = len(shape)
+        g = Grid(dim, shape, (0.3,) * dim, integ, 0.05)
+        r2 = sum(np.reshape(g.axis_r(j) ** 2, [-1 if k == j else 1 for k in range(dim)]) for j in range(dim))
+        g.set_potential(-1.0 / np.sqrt(r2 + 0.5))
+        if masked:
+            for j in range(dim):
+                g.set_mask_axis(j, np.linspace(0.97, 1.0, shape[j]))
+        st = g.state(np.exp(-0.5 * r2) + 0j)
+        A = np.random.default_rng(2).standard_normal((5, g.s, dim)) * 0.05
+        try:
+            g.run_velocity(st, A[:steps])
+            return st.download()
+        finally:
+            g.close()
+
+    want = run(5)
+    for tables in range(1, 12):
+        monkeypatch.setenv("QND_FAIL_TABLES_ABOVE", str(tables))
+        try:
+            run(1)
+            break
+        except QndError as e:
+            assert e.code == 3
+    got = run(5)
+    # the same operators, the factor of a boundary as one product or two
+    assert np.linalg.norm(got - want) <= 1e-13 * np.linalg.norm(want)
