@@ -768,12 +768,15 @@ __device__ __forceinline__ void pass_group(const PassArgs<R>& a, long long g, un
 #pragma unroll
                 for (int u = 0; u < E; ++u) v[u] = cadd(v[u], sum[flat_at(u)]);
             }
-            if (a.dst) {
-#pragma unroll
-                for (int u = 0; u < E; ++u) a.dst[flat_at(u)] = v[u];
-            }
         }
+        // The sums before the store: their partner reads go across the stride of lines that other CTAs share
+        // sectors with, and behind the store they waited for it (two energy moments at 1024^2: 97 us against
+        // 123 in FP32, 118 against 130 in FP64).
         if (a.red.n) reduce();
+        if (active && a.dst) {
+#pragma unroll
+            for (int u = 0; u < E; ++u) a.dst[base + ((long long)(tid + u * T) << log2S)] = v[u];
+        }
     } else {
         // PROPAGATE: one sandwich or two; factors and reductions before the first, between them and after
         // the last
