@@ -869,62 +869,65 @@ __global__ void __launch_bounds__(PassShape<R, L, VAR>::NT, PassShape<R, L, VAR>
 
 // Element-wise reductions over a whole state in r-space (no transform): norm, dipole,
 // acceleration, potential energy of an arbitrary state.
-// Bound by the reads of the state, its partner and the weights: a thread has four points of each on their
-// way at a time. With one point, whose reads the tests of the descriptor put one behind the other,
-// two energy moments at 2^21 points took 219 us in FP32 and 276 in FP64; they take 195 and 249.
+// Bound by the reads of the state, its partner and the weights: a thread has Q points of each on their way
+// at a time, in 64 registers, so that all of the grid's 4 blocks per SM (reduce_blocks) run in one wave. Norm,
+// dipoles and energy in FP32 take, with one, two and four points, 202, 192 and 191 us at 2^21 points and 139, 137
+// and 145 at 1024^2 (code to fetch); with 79 registers, and so a second wave of blocks, 228 and 164.
 template <typename R>
-__global__ void __launch_bounds__(256) qnd_grid_reduce_kernel(const __grid_constant__ PassArgs<R> a, long long n) {
+__global__ void __launch_bounds__(256, 4) qnd_grid_reduce_kernel(const __grid_constant__ PassArgs<R> a, long long n) {
     using V = cplx_t<R>;
-    constexpr int Q = 4;
+    constexpr int Q = 2;
     double acc[MAX_RED];
 #pragma unroll
     for (int k = 0; k < MAX_RED; ++k) acc[k] = 0.0;
-    const int sa = a.shift[a.axis];
-    const long long L = a.nmask[a.axis] + 1;
+    const int sa = a.shift[a.axis], log2L = __popcll(a.nmask[a.axis]);  // lengths are powers of two
     const long long step = (long long)gridDim.x * blockDim.x;
     for (long long i0 = (long long)blockIdx.x * blockDim.x + threadIdx.x; i0 < n; i0 += Q * step) {
-        V v[Q], p[Q];
-        long long at[Q], li[Q];  // the point (past the end: the last one again) and its index in the weights' order
+        // a point past the end reads the last one again and is not added
+        auto at = [&](int q) { return i0 + q * step < n ? i0 + q * step : n - 1; };
+        double abs2[Q], other[Q];  // |v|^2; Re(conj(partner) v), or without a partner the test of RK_NONFINITE
+        {
+            V v[Q];
 #pragma unroll
-        for (int q = 0; q < Q; ++q) {
-            at[q] = i0 + q * step < n ? i0 + q * step : n - 1;
-            v[q] = a.psi[at[q]];
-            li[q] = at[q];
-        }
-        if (a.partner) {
+            for (int q = 0; q < Q; ++q) v[q] = a.psi[at(q)];
+            if (a.partner) {
+                V p[Q];
 #pragma unroll
-            for (int q = 0; q < Q; ++q) p[q] = a.partner[at[q]];
-        }
-        if (a.red_lm) {
+                for (int q = 0; q < Q; ++q) p[q] = a.partner[at(q)];
 #pragma unroll
-            for (int q = 0; q < Q; ++q) {
-                const long long m = (at[q] >> sa) & a.nmask[a.axis];
-                li[q] = ((((at[q] >> sa) / L) << sa) | (at[q] & ((1ll << sa) - 1))) * L + m;
+                for (int q = 0; q < Q; ++q) other[q] = double(p[q].x) * double(v[q].x) + double(p[q].y) * double(v[q].y);
+            } else {
+#pragma unroll
+                for (int q = 0; q < Q; ++q) other[q] = isfinite(double(v[q].x)) && isfinite(double(v[q].y)) ? 0.0 : 1.0;
             }
+#pragma unroll
+            for (int q = 0; q < Q; ++q) abs2[q] = double(v[q].x) * double(v[q].x) + double(v[q].y) * double(v[q].y);
         }
 #pragma unroll
         for (int k = 0; k < MAX_RED; ++k) {
             if (k >= a.red.n) break;
-            double val[Q], w[Q];
-            const int kind = a.red.kind[k], wk = a.red.wkind[k];
+            const bool square = a.red.kind[k] == RK_ABS2;
+            const int wk = a.red.wkind[k];
+            double w[Q];
+            if (wk == WK_ONE) {
 #pragma unroll
-            for (int q = 0; q < Q; ++q) w[q] = 1.0;
-            if (wk == WK_AXIS) {
+                for (int q = 0; q < Q; ++q) w[q] = 1.0;
+            } else {
 #pragma unroll
-                for (int q = 0; q < Q; ++q)
-                    w[q] = __ldg(a.red.wtab[k] + ((at[q] >> a.red.wshift[k]) & a.red.wmask[k]));
-            } else if (wk == WK_GRID) {
-#pragma unroll
-                for (int q = 0; q < Q; ++q) w[q] = __ldg(a.red.wtab[k] + li[q]);
+                for (int q = 0; q < Q; ++q) {
+                    long long li = at(q);
+                    if (wk == WK_AXIS) {
+                        li = (li >> a.red.wshift[k]) & a.red.wmask[k];
+                    } else if (a.red_lm) {  // a full-grid weight in the line-major order of `axis`
+                        const long long m = (li >> sa) & a.nmask[a.axis];
+                        li = ((((li >> sa >> log2L) << sa) | (li & ((1ll << sa) - 1))) << log2L) + m;
+                    }
+                    w[q] = __ldg(a.red.wtab[k] + li);
+                }
             }
 #pragma unroll
-            for (int q = 0; q < Q; ++q) {
-                const double x = v[q].x, y = v[q].y;
-                if (kind == RK_ABS2) val[q] = x * x + y * y;
-                else if (kind == RK_BILIN) val[q] = double(p[q].x) * x + double(p[q].y) * y;
-                else val[q] = isfinite(x) && isfinite(y) ? 0.0 : 1.0;  // RK_NONFINITE
-                if (i0 + q * step < n) acc[k] += val[q] * w[q];
-            }
+            for (int q = 0; q < Q; ++q)
+                if (i0 + q * step < n) acc[k] += (square ? abs2[q] : other[q]) * w[q];
         }
     }
     finish_red<256>(a.red, acc);
