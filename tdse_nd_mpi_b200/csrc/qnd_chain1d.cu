@@ -8,6 +8,8 @@
 // transform, about 2,400 cycles of one SM's FP64 pipe, and its exchanges about 2,000 cycles of its
 // shared memory; two transforms per sandwich. The tables come from L2, read into registers before the
 // transform that precedes their use.
+#include <algorithm>
+
 #include "qnd_kernels.cuh"
 
 #ifndef QND_CHAIN_FP64
@@ -44,8 +46,9 @@ template <typename R, int L, int E> struct ChainShape {
     static constexpr size_t SMEM = sizeof(cplx_t<R>) * (size_t(TW) + P::SMEM_LINE);
 };
 
-template <typename R, int L, int E>
-__global__ void __launch_bounds__(ChainShape<R, L, E>::NT, 1) qnd_chain1d_kernel(const __grid_constant__ Chain1dArgs<R> a) {
+template <typename R, int L, int E, int OPS>
+__global__ void __launch_bounds__(ChainShape<R, L, E>::NT, 1)
+    qnd_chain1d_kernel(const __grid_constant__ Chain1dArgs<R, OPS> a) {
     using V = cplx_t<R>;
     using SH = ChainShape<R, L, E>;
     constexpr int T = SH::T, NT = SH::NT;
@@ -64,11 +67,14 @@ __global__ void __launch_bounds__(ChainShape<R, L, E>::NT, 1) qnd_chain1d_kernel
     const bool counts = t < T;
     const LineSync<T> lsync{1};
 
-    for (int i = t; i < (sizeof(R) == 8 ? SH::P::twb_size() : SH::P::tw_size()); i += NT) tw[i] = a.tw[i];
+    // every twiddle's copy on its way at once: a line of one warp copies up to 30 of them a thread
+    for (int i = t; i < (sizeof(R) == 8 ? SH::P::twb_size() : SH::P::tw_size()); i += NT) cp_async_elem(tw + i, a.tw + i);
+    cp_async_commit();
     V v[E];
 #pragma unroll
     for (int u = 0; u < E; ++u) v[u] = a.src[tid + u * T];
     load_red_rows<NT>(a.red, 0, red_sh);
+    cp_async_wait<0>();
     __syncthreads();  // twiddles and reductions visible
 
     // the point-wise factor `mid` (a full-grid table) with the laser phases at `laser`, the step mask
@@ -162,10 +168,10 @@ __global__ void __launch_bounds__(ChainShape<R, L, E>::NT, 1) qnd_chain1d_kernel
     for (int u = 0; u < E; ++u) a.psi[tid + u * T] = v[u];
 }
 
-template <typename R, int L> static cudaError_t launch_one(const Chain1dArgs<R>& a, cudaStream_t st) {
+template <typename R, int L, int OPS> static cudaError_t launch_args(const Chain1dArgs<R, OPS>& a, cudaStream_t st) {
     constexpr int E = chain1d_values(L, sizeof(R) == 8);
     using SH = ChainShape<R, L, E>;
-    auto* fn = &qnd_chain1d_kernel<R, L, E>;
+    auto* fn = &qnd_chain1d_kernel<R, L, E, OPS>;
     if constexpr (SH::SMEM > 48 * 1024) {
         const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(SH::SMEM));
         if (e != cudaSuccess) return e;
@@ -174,22 +180,37 @@ template <typename R, int L> static cudaError_t launch_one(const Chain1dArgs<R>&
     return cudaGetLastError();
 }
 
-template <typename R> cudaError_t launch_chain1d(int L, const Chain1dArgs<R>& a, cudaStream_t st) {
+template <typename R, int L, int OPS>
+static cudaError_t launch_ops(const Chain1dHead<R>& head, const Chain1dOp* ops, cudaStream_t st) {
+    Chain1dArgs<R, OPS> a;
+    static_cast<Chain1dHead<R>&>(a) = head;
+    std::copy(ops, ops + head.nops, a.ops);
+    return launch_args<R, L>(a, st);
+}
+
+template <typename R, int L>
+static cudaError_t launch_one(const Chain1dHead<R>& head, const Chain1dOp* ops, cudaStream_t st) {
+    static_assert(sizeof(Chain1dArgs<R, CHAIN1D_SHORT>) <= 4096, "the short list's arguments");
+    return head.nops <= CHAIN1D_SHORT ? launch_ops<R, L, CHAIN1D_SHORT>(head, ops, st)
+                                      : launch_ops<R, L, CHAIN1D_OPS>(head, ops, st);
+}
+
+template <typename R> cudaError_t launch_chain1d(int L, const Chain1dHead<R>& a, const Chain1dOp* ops, cudaStream_t st) {
     switch (L) {
-    case 128: return launch_one<R, 128>(a, st);
-    case 256: return launch_one<R, 256>(a, st);
-    case 512: return launch_one<R, 512>(a, st);
-    case 1024: return launch_one<R, 1024>(a, st);
-    case 2048: return launch_one<R, 2048>(a, st);
-    case 4096: return launch_one<R, 4096>(a, st);
+    case 128: return launch_one<R, 128>(a, ops, st);
+    case 256: return launch_one<R, 256>(a, ops, st);
+    case 512: return launch_one<R, 512>(a, ops, st);
+    case 1024: return launch_one<R, 1024>(a, ops, st);
+    case 2048: return launch_one<R, 2048>(a, ops, st);
+    case 4096: return launch_one<R, 4096>(a, ops, st);
     default: return cudaErrorInvalidValue;
     }
 }
 
 #if QND_CHAIN_FP64
-template cudaError_t launch_chain1d<double>(int, const Chain1dArgs<double>&, cudaStream_t);
+template cudaError_t launch_chain1d<double>(int, const Chain1dHead<double>&, const Chain1dOp*, cudaStream_t);
 #else
-template cudaError_t launch_chain1d<float>(int, const Chain1dArgs<float>&, cudaStream_t);
+template cudaError_t launch_chain1d<float>(int, const Chain1dHead<float>&, const Chain1dOp*, cudaStream_t);
 #endif
 
 }  // namespace qnd

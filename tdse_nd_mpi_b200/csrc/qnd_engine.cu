@@ -1832,13 +1832,15 @@ static void run_chain1d(qnd_ctx* c, void* psi, const std::vector<ChainK>& K, con
     auto run = [&](auto tag) {
         using R = decltype(tag);
         using V = cplx_t<R>;
-        auto ap = std::make_unique<Chain1dArgs<R>>();
-        Chain1dArgs<R>& a = *ap;
+        Chain1dHead<R> a;
+        std::vector<Chain1dOp> ops;
+        ops.reserve(size_t(std::min<int64_t>(NK, CHAIN1D_OPS)));
         const V* field = static_cast<const V*>(c->field_view ? c->field_view : c->field_tab.p);
         std::vector<ChainK> specs;     // distinct tables of the launch being filled
         std::vector<Factor> mids;
         auto begin = [&]() {
-            a = Chain1dArgs<R>{};
+            a = Chain1dHead<R>{};
+            ops.clear();
             a.psi = static_cast<V*>(psi);
             a.src = src ? static_cast<const V*>(src) : a.psi;
             src = nullptr;  // a later launch goes on from psi
@@ -1878,7 +1880,8 @@ static void run_chain1d(qnd_ctx* c, void* psi, const std::vector<ChainK>& K, con
         auto launch = [&]() {
             a.seed = uint32_t(c->kernels_launched) * 0x9e3779b9u + 0x632be5abu;
             const auto ev = profile_begin(c);
-            QND_CK(launch_chain1d<R>(int(c->nr[0]), a, c->stream));
+            a.nops = int(ops.size());
+            QND_CK(launch_chain1d<R>(int(c->nr[0]), a, ops.data(), c->stream));
             c->kernels_launched++;
             profile_end(c, ev);
         };
@@ -1887,12 +1890,13 @@ static void run_chain1d(qnd_ctx* c, void* psi, const std::vector<ChainK>& K, con
         if (pre.laser_ia >= 0) a.pre_laser = laser_at(pre_lst, pre.laser_ia);
         a.pre_scale = pre_scale;
         for (int64_t i = 0; i < NK; ++i) {
-            if (a.nops == CHAIN1D_OPS || specs.size() + 1 > CHAIN1D_TABLES || mids.size() + 2 > CHAIN1D_TABLES) {
+            if (ops.size() == size_t(CHAIN1D_OPS) || specs.size() + 1 > CHAIN1D_TABLES || mids.size() + 2 > CHAIN1D_TABLES) {
                 launch();
                 begin();
             }
             const ChainMid& m = i + 1 < NK ? M[i] : post;
-            Chain1dOp& op = a.ops[a.nops++];
+            ops.emplace_back();
+            Chain1dOp& op = ops.back();
             if (K[i].kind == KV_FIELD) op.field_spec = laser_at(K[i].lst, K[i].ia);
             else op.spec = spec_id(K[i]);
             op.mid = mid_id(m.f);

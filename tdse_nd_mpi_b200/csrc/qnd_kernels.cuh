@@ -218,6 +218,10 @@ template <typename R> void launch_apply_combine(long long n, cplx_t<R>* dst, con
 
 // ---- 1-D grids of up to 4096 points: a chain of sandwiches in one launch (qnd_chain1d.cu)
 constexpr int CHAIN1D_OPS = 512;     // sandwiches per launch (longer chains take several launches)
+// Launches of up to this many carry a shorter list, which keeps their arguments below 4 KB. With the long
+// list (12 KB) a call of one Verlet step in imaginary time took 20 us at 512 FP32 points and takes 15.4,
+// at 128 FP64 points 22 and 17 (in FP32 half of that are the twiddles' copies, see the kernel).
+constexpr int CHAIN1D_SHORT = 120;
 constexpr int CHAIN1D_TABLES = 24;   // distinct spectral / r-space tables per launch
 // Line lengths the chain kernel is built for, and its values per thread.
 // FP32 keeps the pass kernels' 16 at every length, with them their stages and their roundings: with 8 (a
@@ -236,7 +240,7 @@ struct Chain1dOp {
     int laser = -1;       // field-table offset of the laser phases
     int obs = -1;
 };
-template <typename R> struct Chain1dArgs {
+template <typename R> struct Chain1dHead {
     using V = cplx_t<R>;
     V* psi;
     const V* src;         // where the state is read (psi, or another state that stays)
@@ -255,9 +259,11 @@ template <typename R> struct Chain1dArgs {
     int* gs_flag;
     double dNr, gs_tol;
     int nops;
-    Chain1dOp ops[CHAIN1D_OPS];
 };
-template <typename R> cudaError_t launch_chain1d(int L, const Chain1dArgs<R>& a, cudaStream_t st);
+template <typename R, int OPS> struct Chain1dArgs : Chain1dHead<R> {
+    Chain1dOp ops[OPS];
+};
+template <typename R> cudaError_t launch_chain1d(int L, const Chain1dHead<R>& a, const Chain1dOp* ops, cudaStream_t st);
 
 // ---- the persistent sweep kernel (qnd_sweep.cu): recorded passes of many members in one launch
 constexpr int SWEEP_NT = 128;  // threads per CTA: every line length it takes has 128-thread pass CTAs

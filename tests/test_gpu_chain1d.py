@@ -79,3 +79,22 @@ def test_imaginary_time_states(qnd_lib, n, precision, tol):
         o.imag_state(want, j, steps)
         g.imag_propagate(states, j, steps)
         assert rel(states[j].download(), want[j]) < tol
+
+
+@pytest.mark.parametrize("n", [128, 4096])
+@pytest.mark.parametrize("precision,tol", [("fp64", 5e-15), ("mixed", 3e-6)])
+@pytest.mark.parametrize("steps", [119, 120, 511, 512])
+def test_lists_of_sandwiches(qnd_lib, n, precision, tol, steps):
+    """The last short and first long list of a launch (Verlet: steps + 1 sandwiches), the last list of one
+    launch and the first of two: the run in one call equals the run in two halves, whose boundary rounds
+    the state's factors once more (FP32: the dithered roundings of a launch differ, a random walk of
+    2^-24 over two transforms of up to 12 levels a step, seven times that allowed)."""
+    g, _ = _pair(n, "Verlet", precision)
+    psi0 = O.smooth_state((n,), DR, 4)
+    F = np.random.default_rng(steps).standard_normal((steps, 1, 1)) * 0.05
+    one, two = g.state(psi0), g.state(psi0)
+    g.run_length(one, F)
+    g.run_length(two, F[:steps // 2])
+    g.run_length(two, F[steps // 2:])
+    assert rel(two.download(), one.download()) <= tol * np.sqrt(steps)
+    g.close()
