@@ -186,6 +186,33 @@ template <typename R, int L, int VAR = 0> struct PassShape {
     __host__ __device__ static constexpr int line_off(int w) {
         return w * LS + (T < SLOTS ? w / (SLOTS / T) % T : 0);
     }
+    // What LS and line_off are chosen for, checked where a shape is built (qnd_pass_inst.cu): no line reaches
+    // into the next one or past the buffer, and ...
+    static constexpr bool lines_apart() {
+        for (int w = 0; w < G; ++w)
+            if (line_off(w) + FFTPlan<L, E>::SMEM_LINE > (w + 1 < G ? line_off(w + 1) : G * LS)) return false;
+        return true;
+    }
+    // ... for lines of fewer threads than a bank cycle has slots, the accesses of one bank cycle fall on
+    // distinct slots: an exchange's store of register r by the threads of SLOTS / T lines, and the staging
+    // copy's SLOTS neighbouring lines.
+    static constexpr bool slots_distinct() {
+        if (T >= SLOTS || G < SLOTS) return true;
+        constexpr int Q = T < SLOTS ? SLOTS / T : 1;
+        for (int w0 = 0; w0 + Q <= G; w0 += Q)
+            for (int r = 0; r < E; ++r) {
+                unsigned hit = 0;
+                for (int w = w0; w < w0 + Q; ++w)
+                    for (int t = 0; t < T; ++t) hit |= 1u << (line_off(w) + (E * t + r) + (E * t + r) / E) % SLOTS;
+                if (hit != (1u << SLOTS) - 1) return false;
+            }
+        for (int w0 = 0; w0 + SLOTS <= G; w0 += SLOTS) {
+            unsigned hit = 0;
+            for (int w = w0; w < w0 + SLOTS; ++w) hit |= 1u << line_off(w) % SLOTS;
+            if (hit != (1u << SLOTS) - 1) return false;
+        }
+        return true;
+    }
     // stage twiddle entries: FP64 plans keep one base per butterfly position (TwiddledDFT)
     static constexpr int TW_ENTRIES = sizeof(R) == 8 ? FFTPlan<L, E>::twb_size() : FFTPlan<L, E>::tw_size();
     static constexpr int TWN_RAW = (TW_ENTRIES + 1) & ~1;

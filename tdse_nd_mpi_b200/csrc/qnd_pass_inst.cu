@@ -18,6 +18,7 @@ template <typename R, int L, int VAR> static PassKernelInfo variant_info(int sk,
     using SH = PassShape<R, L, VAR>;
     const void* fn = nullptr;
     if constexpr (SH::VALID) {
+        static_assert(SH::lines_apart() && SH::slots_distinct(), "the layout of a CTA's lines");
 #define QND_PICKV(M) QND_SK(R, L, M, VAR)
         switch (mode) {
         case PM_SANDWICH: fn = QND_PICKV(PM_SANDWICH); break;
@@ -35,6 +36,7 @@ template <typename R, int L> PassKernelInfo pass_kernel_info(bool strided, int m
     if (var == 2) return variant_info<R, L, 2>(sk, mode);
     if (var == 3) return variant_info<R, L, 3>(sk, mode);
     using SH = PassShape<R, L>;
+    static_assert(SH::lines_apart() && SH::slots_distinct(), "the layout of a CTA's lines");
     const void* fn = nullptr;
 #define QND_PICK(M) QND_SK(R, L, M, 0)
     switch (mode) {
