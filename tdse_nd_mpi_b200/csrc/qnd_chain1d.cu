@@ -6,8 +6,8 @@
 //
 // What bounds it: one SM. A line of 4096 FP64 points needs 588 FP64 instructions per 16 points and
 // transform, about 2,400 cycles of one SM's FP64 pipe, and its exchanges about 2,000 cycles of its
-// shared memory; two transforms per sandwich. The tables come from L2, read into registers before the
-// transform that precedes their use.
+// shared memory; two transforms per sandwich. The tables come from L2: the spectral row is read into
+// registers during the forward transform, the r-space factors one table after the other after the inverse.
 #include <algorithm>
 
 #include "qnd_kernels.cuh"

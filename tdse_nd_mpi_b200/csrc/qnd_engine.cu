@@ -907,6 +907,9 @@ static void load_shape_table() {
 }
 
 static int shape_choice(qnd_ctx* c, const PassSpec& ps, int L, int log2S) {
+    // Passes at a chain's ends in the momentum representation (one or two per call and axis) are built in the
+    // default shape only: with every shape one BM4 step a call took 163 us against 166 at 1024^2 in FP64,
+    // 123.4 against 124.4 in mixed precision, and the same to 1% from 256^2 to 256 x 2048.
     const int mode = ps.mode, kmode = pass_kernel_mode(mode, ps.red.n > 0);
     if (ps.vL || ps.from_p || ps.to_p || (mode != PM_SANDWICH && mode != PM_DOUBLE) || L < 256 || L > 2048) return 0;
     const bool strided = log2S > 0;
@@ -1816,8 +1819,8 @@ static int chain_final_axis(const qnd_ctx* c, int NK) { return sandwich_last_axi
 // 1-D grids whose chains run in one launch of the chain kernel (qnd_chain1d.cu): lengths of 128 to 4096
 // points. A pass of such a grid is one CTA on one SM, so a launch per pair of sandwiches left the GPU
 // waiting on launches and on the state's round trip: a BM4 step took 77 us at 4096 points (with
-// Gram-Schmidt) and 34 us at 512 (with observables) by passes, and takes 37 and 12.7 us by this kernel. Shorter lines have fewer than a warp of
-// 4-point threads and keep the passes.
+// Gram-Schmidt) and 34 us at 512 (with observables) by passes, and takes 37 and 12.7 us by this kernel.
+// Shorter lines have fewer than a warp of 4-point threads and keep the passes.
 static bool chain1d(const qnd_ctx* c) { return c->tw_chain.p && !c->recorder; }
 
 struct ChainGs {
@@ -1922,16 +1925,7 @@ static void run_chain1d(qnd_ctx* c, void* psi, const std::vector<ChainK>& K, con
     else run(float{});
 }
 
-// Run a chain of kinetic sandwiches K_0 .. K_{NK-1} with M[i] between K_i and K_{i+1}, `pre` (and
-// the device scalar pre_scale) before K_0 and `post` after K_{NK-1}. Consecutive sandwiches run
-// their axes in opposite orders, so the last axis of K_i is the first axis of K_{i+1}: those two
-// axis passes and M[i] fuse into one PM_DOUBLE pass. A chain of NK sandwiches costs NK + 1 passes
-// in 2-D (2 NK + 1 in 3-D) instead of d NK; in 1-D the sandwiches pair up two per pass, and a
-// factor between pairs moves into the next pass's prologue (1-D chains carry no mask or
-// reductions between sandwiches).
-// from_p / to_p: psi is in the unitary momentum representation before K_0 / after K_{NK-1} (chain_ends_in_p
-// says where; pre and post are then empty): the passes of those sandwiches leave out the transform that
-// the change of representation would undo, which saves its d passes.
+// Whether a chain may begin or end in the unitary momentum representation (run_chain's from_p, to_p).
 static bool chain_ends_in_p(const qnd_ctx* c) {
     if (c->dim < 2 || c->recorder) return false;
     for (int j = 0; j < c->dim; ++j)
@@ -1943,6 +1937,16 @@ static void copy_state(qnd_ctx* c, void* dst, const void* src) {
     QND_CK(cudaMemcpyAsync(dst, src, size_t(c->n) * c->elem(), cudaMemcpyDeviceToDevice, c->stream));
 }
 
+// Run a chain of kinetic sandwiches K_0 .. K_{NK-1} with M[i] between K_i and K_{i+1}, `pre` (and
+// the device scalar pre_scale) before K_0 and `post` after K_{NK-1}. Consecutive sandwiches run
+// their axes in opposite orders, so the last axis of K_i is the first axis of K_{i+1}: those two
+// axis passes and M[i] fuse into one PM_DOUBLE pass. A chain of NK sandwiches costs NK + 1 passes
+// in 2-D (2 NK + 1 in 3-D) instead of d NK; in 1-D the sandwiches pair up two per pass, and a
+// factor between pairs moves into the next pass's prologue (1-D chains carry no mask or
+// reductions between sandwiches).
+// from_p / to_p: psi is in the unitary momentum representation before K_0 / after K_{NK-1} (where chain_ends_in_p
+// says so; pre and post are then empty): the passes of those sandwiches leave out the transform that
+// the change of representation would undo, which saves its d passes.
 static void run_chain(qnd_ctx* c, void* psi, const std::vector<ChainK>& K, const std::vector<ChainMid>& M,
                       const Factor& pre, int64_t pre_lst, const double* pre_scale, const ChainMid& post,
                       bool from_p = false, bool to_p = false, const void* src = nullptr) {
@@ -2949,12 +2953,15 @@ static void build_long_axis_nd(qnd_ctx* c, int ax) {
 static void build_long_axis(qnd_ctx* c) {
     const int64_t N = c->nr[0];
     c->long1d = true;
-    // FP64: two lengths of about the same size (the shorter one strided), 64 to 4096 points each: both
-    // virtual axes then have many lines to spread over the SMs (64 x 4096 gave the contiguous pass of
-    // 262144 points 64 CTAs for 148 SMs, 29.6 us). From 2^16 to 2^18 points the contiguous axis takes 256
-    // points, two radix-16 stages. us per BM4 step with observables: 2^17 as 512 x 256 101, as 256 x 512
-    // 108; 2^18 as 1024 x 256 117, as 512 x 512 122, as 256 x 1024 125; 2^19 as 512 x 1024 172, as
-    // 2048 x 256 181; 2^20 as 1024 x 1024 276, as 4096 x 256 477.
+    // FP64: two lengths of about the same size, 64 to 4096 points each, so that both virtual axes have many
+    // lines to spread over the SMs (64 x 4096 gave the contiguous pass of 262144 points 64 CTAs for 148 SMs,
+    // 29.6 us). From 2^16 to 2^18 points the contiguous length is 256, two radix-16 stages, and the strided
+    // one the rest, which may be the longer. us per BM4 step with observables, by the logarithm of the strided
+    // length (the rule's choice in brackets):
+    //   2^13  4: 90, 5: 84, [6: 87], 7: 95     2^16  7: 105, [8: 91], 9: 97     2^19  8: 172, [9: 175], 10: 169
+    //   2^14  5: 90, 6: 90, [7: 96], 8: 97     2^17  8: 107, [9: 107], 10: 107  2^20  9: 289, [10: 284], 11: 299
+    //   2^15  5: 94, 6: 96, [7: 98], 8: 98     2^18  8: 121, 9: 124, [10: 121]  2^21  9: 873, [10: 554], 11: 595
+    //   2^22  10: 1609, [11: 1113], 12: 1720
     // FP32: the split also sets the rounding. 16 points strided up to 2^15 and 256 after (up to 4096
     // contiguous) are the fastest splits whose errors against 64 bits stay those of n2 = 4096: after 16
     // imaginary-time steps 8192 points are 2.5e-6 off as 16 x 512 and 4.0e-6 as 64 x 128, 131072 9.4e-6 as

@@ -227,7 +227,8 @@ constexpr int CHAIN1D_TABLES = 24;   // distinct spectral / r-space tables per l
 // FP32 keeps the pass kernels' 16 at every length, with them their stages and their roundings: with 8 (a
 // stage more, and twice the dithered factors) a 256-point run was twice as far from 64-bit results.
 // Measured with FP64, us per BM4 step with observables: 512 points 12.7 with 8 values (4: 16.6, 16: 19.1),
-// 1024 19.1 (16: 21.4), 2048 27.7 with 16 (8: 29.6), 4096 (imaginary time) 37 with 16 (8: 44).
+// 1024 19.1 (16: 21.4), 2048 27.7 with 16 (8: 29.6), 4096 (imaginary time) 37 with 16 (8: 44); in calls of
+// eight steps 128 points 16.4 with 4 (8: 18.0, 16: 20.7), 256 19.1 with 8 (4: 17.6, 16: 22.4).
 constexpr bool chain1d_length_ok(long long L) { return L >= 128 && L <= 4096 && (L & (L - 1)) == 0; }
 constexpr int chain1d_values(int L, bool fp64) { return !fp64 ? 16 : (L == 128 ? 4 : (L < 2048 ? 8 : 16)); }
 // One sandwich and the point-wise work after it, in this order: factor `mid` with the laser phases and

@@ -697,18 +697,18 @@ __device__ __forceinline__ void pass_group(const PassArgs<R>& a, long long g, un
         for (int u = 0; u < E; ++u)
             v[u] = fmul_spec<L>(v[u], __ldg(row + tid + u * T), key + uint32_t(tid + u * T), u == 0 || u == E - 1);
     };
-    // v <- IFFT[ between . FFT v ]. ONE_TRANSFORM: one copy of the transform, the inverse as the forward
-    // transform of the conjugate, conjugated: less code to fetch against two sign flips per point.
-    // Measured with one copy / with two, FP64: 2048^2 6.73 / 7.09 ms, 1024^2 7.48 / 7.51, 3-D grids of 64
-    // to 256 points 2.74 / 2.66. FP32 passes keep both directions: 2048^2 13.2 / 12.5 ms, and the low parts
-    // of their split constants round differently in the conjugate (the sweep of 256^2 to 1024^2 members
-    // would gain 3%).
     auto second_mid = [&] {
         if (active && a.mid2_cplx) {
 #pragma unroll
             for (int u = 0; u < E; ++u) v[u] = fmul(v[u], __ldg(a.mid2_cplx + lbase + tid + u * T));
         }
     };
+    // v <- IFFT[ between . FFT v ]. ONE_TRANSFORM: one copy of the transform, the inverse as the forward
+    // transform of the conjugate, conjugated: less code to fetch against two sign flips per point.
+    // Measured with one copy / with two, FP64: 2048^2 6.73 / 7.09 ms, 1024^2 7.48 / 7.51, 3-D grids of 64
+    // to 256 points 2.74 / 2.66. FP32 passes keep both directions: 2048^2 13.2 / 12.5 ms, and the low parts
+    // of their split constants round differently in the conjugate (the sweep of 256^2 to 1024^2 members
+    // would gain 3%).
     // fwd / inv: whether the transforms run (PassArgs from_p, to_p).
     auto sandwich = [&](bool fwd, bool inv, auto between) {
         if constexpr (ONE_TRANSFORM) {

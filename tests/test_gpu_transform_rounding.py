@@ -29,3 +29,20 @@ def test_unitary_transform_rounding(qnd_lib, n, axis):
     # the largest single error, against the largest value's size
     assert np.max(np.abs(got - want)) <= 32 * levels * 2.0**-53 * np.max(np.abs(want))
     grid.close()
+
+
+@pytest.mark.parametrize("n", [16, 32, 256, 512, 1024, 4096])
+@pytest.mark.parametrize("axis", [0, 1])
+def test_transform_rounding_is_the_expected_walk(qnd_lib, n, axis):
+    """Three times the expected error: about two units in the last place per butterfly level (the factor,
+    formed by up to three squarings, and the sum), adding up as a random walk over the levels."""
+    from tdse_nd_mpi_b200 import Grid
+
+    shape = (n, 32) if axis == 0 else (32, n)
+    grid = Grid(2, shape, (0.2, 0.3), "Verlet", 0.05)
+    psi = O.seeded_state(shape, 3 * n + axis)
+    st = grid.state(psi)
+    grid.to_p(st)
+    want = np.fft.fftn(psi, norm="ortho")
+    assert np.linalg.norm(st.download() - want) <= 6 * np.sqrt(np.log2(n) + 5) * 2.0**-53 * np.linalg.norm(want)
+    grid.close()
