@@ -36,3 +36,15 @@ def test_shape_table_lines_are_valid():
         key = (prec, n, L, log2S, kind)
         assert key not in seen, l
         seen.add(key)
+
+
+def test_every_shape_is_timed():
+    """A row holds one time per shape: a row with fewer was measured on kernels of an earlier build."""
+    with open(TABLE) as f:
+        rows = [LINE.match(l.rstrip("\n")) for l in f if l.strip() and not l.startswith("#")]
+    assert rows
+    for m in rows:
+        times = [float(x) for x in m.group(6).split(",")]
+        assert len(times) == 4, m.group(0)
+        L = int(m.group(3))
+        assert times[0] > 0 and times[2] > 0 and (times[1] > 0) == (L < 2048) and (times[3] > 0) == (L == 1024), m.group(0)
