@@ -3983,17 +3983,21 @@ int qnd_run_length_sweep(int count, qnd_ctx* const* ctxs, void* const* psi_r_dev
     int failed = 0;
     for (int64_t s0 = 0; s0 < nsteps && !failed; s0 += SWEEP_SEGMENT) {
         const int64_t seg = std::min(SWEEP_SEGMENT, nsteps - s0);
-        // record every member's chains for this segment (their field tables built on their streams), or
-        // launch them (1-D members)
+        // record every member's chains for this segment (their field tables built on their streams), then
+        // launch those of the 1-D members (last: an error while recording leaves every state as it was)
         std::vector<std::vector<RecordedPass>> rec(static_cast<size_t>(count));
-        int ndirect = 0;
-        for (int i = 0; i < count; ++i) {
+        std::vector<int> order;
+        for (int i = 0; i < count; ++i)
+            if (!chain1d(ctxs[i])) order.push_back(i);
+        const int ndirect = count - int(order.size());
+        for (int i = 0; i < count; ++i)
+            if (chain1d(ctxs[i])) order.push_back(i);
+        for (int i : order) {
             SweepMember& m = ms[i];
             qnd_ctx* c = m.c;
             const int64_t chunk = chunk_steps(c);
             const size_t per_step = size_t(c->s) * c->axtot * c->elem();
             const bool direct = chain1d(c);
-            ndirect += direct;
             c->sweep_field.ensure(size_t(seg) * per_step);
             for (int64_t c0 = 0; c0 < seg; c0 += chunk) {
                 const int64_t ch = std::min(chunk, seg - c0);
