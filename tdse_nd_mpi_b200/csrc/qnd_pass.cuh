@@ -320,8 +320,8 @@ template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile(
 
 // A fused reduction's accumulators in shared memory, where they are indexed at run time: the loop over
 // them is rolled. With a copy of the sums for each of the MAX_RED accumulators and each weight kind, a
-// reducing 1024-point pass held 175 KB (FP64) to 232 KB (FP32) of code, and a launch finds the
-// instruction caches cold.
+// reducing 1024-point pass held up to 190 KB (FP64) and 237 KB (FP32) of code (64 and 81 KB now), and a
+// launch finds the instruction caches cold.
 struct RedRow {
     const double* w;  // weights: none (null), one for the line at w[(base >> shift) & mask], or a row
     long long mask;
@@ -727,7 +727,7 @@ __device__ __forceinline__ void pass_group(const PassArgs<R>& a, long long g, un
     };
 
     // A pass loops over one copy of the factors and reductions, at the places before, between and after
-    // its sandwiches. A launch finds the instruction caches cold: with a copy per place, 64 KB of code in
+    // its sandwiches. A launch finds the instruction caches cold: with a copy per place, 71 KB of code in
     // the FP64 1024-point two-sandwich pass (30 KB now), its first transforms took 3,500 cycles each more
     // than the second ones of the same launch.
     bool store_out = false;  // write v back to psi at the end
